@@ -387,108 +387,6 @@ __global__ void __launch_bounds__(kTileA * kTileA) k_vjp(VjpArgs<R> a,
 }
 
 // -------------------------------------------------------------------------
-// Adjoint block smoother fused with the update lambda -= omega * delta
-// (vanka.cu:663-797 plus glide/operators.py:517-524).  The local matrix is
-// the forward one at the (fixed) forward state; the tile layout is the
-// forward sweep's, so each block owns its faces and updates lambda in place.
-// -------------------------------------------------------------------------
-template <class R>
-struct AdjSweepArgs {
-    Arr<R> u, v, H, phi, mask, bed, B, beta;
-    Arr<R> ru, rv, rH;     // adjoint residual
-    Arr<R> lu, lv, lH;     // updated in place
-    PhysR<R> p;
-    R omega, ssa_damping, mc_damping;
-    int ny, nx;
-};
-
-// TR = true: adjoint block smoother (solve with J^T; pinned rows get a zero
-// right-hand side, as the reference does).  TR = false: the same smoother for
-// the tangent system J e = f of the binary64 Newton outer iteration, whose
-// pinned rows are identity rows (the correction there equals the residual).
-template <class R, bool TR>
-__global__ void __launch_bounds__(kSweepThreads) k_adjoint_sweep(AdjSweepArgs<R> a) {
-    using TileT = Tile<R, kTile, 2, 1>;
-    constexpr int NC = TileT::NC;
-    constexpr int ND = kTile + 1;
-    __shared__ TileT t;
-    __shared__ R dl[ND][ND][4];
-    const int i0 = blockIdx.y * kTile, j0 = blockIdx.x * kTile;
-    const int ny = a.ny, nx = a.nx;
-    stage_tile<R, kTile, 2, 1>(t, i0, j0, ny, nx, a.u, a.v, a.H, a.bed, a.beta, &a.phi);
-    __syncthreads();
-    TileView<R, kTile, 2, 1> s{t, i0, j0, ny, nx};
-    for (int k = threadIdx.x; k < NC * NC; k += blockDim.x) {
-        int r = k / NC, c = k % NC;
-        int gi = i0 - 2 + r, gj = j0 - 2 + c;
-        R Bc = a.B.at(clampi(gi, 0, ny - 1), clampi(gj, 0, nx - 1));
-        t.eta[r][c] = eta_at<R>(s, Bc, a.p, gi, gj);
-    }
-    __syncthreads();
-    int i, j;
-    const int tid = threadIdx.x;
-    if (tid < kTile * kTile) { i = i0 + tid / kTile; j = j0 + tid % kTile; }
-    else if (tid < kTile * kTile + kTile) { i = i0 + (tid - kTile * kTile); j = j0 - 1; }
-    else { i = i0 - 1; j = j0 + (tid - kTile * kTile - kTile); }
-    const bool live = i >= 0 && i < ny && j >= 0 && j < nx;
-    // the owned cells' unknowns, loaded with the factors rather than after the
-    // barrier (only this thread writes them)
-    const bool own = tid < kTile * kTile && live;
-    R xu0 = R(0), xv0 = R(0), xh0 = R(0);
-    if (own) {
-        xu0 = a.xu.at(i, j);
-        xv0 = a.xv.at(i, j);
-        xh0 = a.xH.at(i, j);
-    }
-    R d4 = 0;
-    R dd[4] = {0, 0, 0, 0};
-    if (live) {
-        R x[5] = {s.U(i, j), s.U(i, j + 1), s.V(i, j), s.V(i + 1, j), s.Hc(i, j)};
-        R J[25], rr[5], JT[25], b[5], dlam[5];
-        local_system<R>(s, a.p, i, j, x, J, rr);
-        J[0] -= a.ssa_damping; J[6] -= a.ssa_damping; J[12] -= a.ssa_damping; J[18] -= a.ssa_damping;
-        J[24] += a.mc_damping;
-        b[0] = a.ru.at(i, j); b[1] = a.ru.at(i, j + 1); b[2] = a.rv.at(i, j); b[3] = a.rv.at(i + 1, j);
-        b[4] = a.rH.at(i, j);
-        const R zpin = R(0);
-        if (j == 0) { pin(J, 0); b[0] = TR ? zpin : b[0]; }
-        if (j == nx - 1) { pin(J, 1); b[1] = TR ? zpin : b[1]; }
-        if (i == 0) { pin(J, 2); b[2] = TR ? zpin : b[2]; }
-        if (i == ny - 1) { pin(J, 3); b[3] = TR ? zpin : b[3]; }
-        if (a.mask.at(i, j) > R(0.5)) { pin(J, 4); b[4] = TR ? zpin : b[4]; }
-        if (TR) {
-#pragma unroll
-            for (int r = 0; r < 5; ++r)
-#pragma unroll
-                for (int c = 0; c < 5; ++c) JT[r * 5 + c] = J[c * 5 + r];
-            lu5_solve(JT, b, dlam);
-        } else {
-            lu5_solve(J, b, dlam);
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) dd[q] = R(0.5) * dlam[q];
-        d4 = dlam[4];
-    }
-    {
-        const int di = i - (i0 - 1), dj = j - (j0 - 1);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) dl[di][dj][q] = dd[q];
-    }
-    __syncthreads();
-    if (tid < kTile * kTile && live) {
-        const int di = i - (i0 - 1), dj = j - (j0 - 1);
-        const R w = a.omega;
-        R du = (j > 0 ? dl[di][dj - 1][1] : R(0)) + dl[di][dj][0];
-        a.lu.at(i, j) = a.lu.at(i, j) - w * du;
-        if (j == nx - 1) a.lu.at(i, nx) = a.lu.at(i, nx) - w * dl[di][dj][1];
-        R dv = (i > 0 ? dl[di - 1][dj][3] : R(0)) + dl[di][dj][2];
-        a.lv.at(i, j) = a.lv.at(i, j) - w * dv;
-        if (i == ny - 1) a.lv.at(ny, j) = a.lv.at(ny, j) - w * dl[di][dj][3];
-        a.lH.at(i, j) = a.lH.at(i, j) - w * d4;
-    }
-}
-
-// -------------------------------------------------------------------------
 // Block factors of the linear smoothers.  During a linear solve the state is
 // fixed, so each cell's 5x5 block (local Newton matrix + damping, pinned
 // rows, transposed for the adjoint) is factored once per V-cycle and stored:
@@ -619,6 +517,8 @@ __global__ void __launch_bounds__(kTile * kTile)
 // One linear block-smoother sweep with stored factors: x += omega * delta
 // with delta = B^-1 (f - Op x) per cell, face corrections averaged between
 // the two cells of a face (adjoint: lambda -= omega * B^-T r, r = J^T lambda - f).
+constexpr int kSweepThreads = kTile * kTile + 2 * kTile;
+
 template <class R, bool TR, class BLK>
 __device__ __forceinline__ void block_sweep_tile(const BlockArgs<R>& a, BLK blk) {
     constexpr int ND = kTile + 1;

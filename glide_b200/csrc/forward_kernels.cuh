@@ -1,6 +1,7 @@
 // forward_kernels.cuh -- residual, fused Vanka sweep and grounding kernels.
 #pragma once
 
+#include "local_cell.cuh"
 #include "stencil.cuh"
 #include "tile.cuh"
 #include "tma.cuh"
@@ -57,14 +58,14 @@ __global__ void __launch_bounds__(256) k_residual(ResidualArgs<R> a,
 // -------------------------------------------------------------------------
 template <class R>
 __global__ void __launch_bounds__(256) k_vanka_dump(ResidualArgs<R> a, R* Jout, R* rout) {
-    using TileT = Tile<R, kTile, 1, 1>;
+    using TileT = Tile<R, kTile, kTile, 1, 1>;
     constexpr int NC = TileT::NC;
     __shared__ TileT t;
     const int i0 = blockIdx.y * kTile, j0 = blockIdx.x * kTile;
     const int ny = a.ny, nx = a.nx;
-    stage_tile<R, kTile, 1, 1>(t, i0, j0, ny, nx, a.u, a.v, a.H, a.bed, a.beta, &a.phi);
+    stage_tile<R, kTile, kTile, 1, 1>(t, i0, j0, ny, nx, a.u, a.v, a.H, a.bed, a.beta, &a.phi);
     __syncthreads();
-    TileView<R, kTile, 1, 1> s{t, i0, j0, ny, nx};
+    TileView<R, kTile, kTile, 1, 1> s{t, i0, j0, ny, nx};
     for (int k = threadIdx.x; k < NC * NC; k += blockDim.x) {
         int r = k / NC, c = k % NC;
         int gi = i0 - 1 + r, gj = j0 - 1 + c;
@@ -175,27 +176,26 @@ struct SweepArgs {
     R relax;                     // local Newton step length (the reference fixes 0.5)
     int newton_steps;
     int ny, nx;
-    int gmode;                   // GammaMode of grouped launches (the kernel's template fixes it)
+    int gmode;                   // GammaMode
 };
 
-constexpr int kSweepThreads = kTile * kTile + 2 * kTile;
-
-// MINB = resident blocks per SM the register allocation is fitted to: 1
-// keeps every value in registers, 2 doubles the warps that hide the FP64
-// dependency latency at the price of some spills; the runtime picks one.
-template <class R, bool PHI_LIVE, class BLK>
+// LIN: the local iteration of local_cell.cuh (linear sliding); otherwise the
+// general local system.  A block of BY x BX threads solves one cell each: its
+// own (BY - 1) x (BX - 1) cells and, redundantly, the row above and the column
+// left of them, so that it owns its faces outright.
+template <class R, bool PHI_LIVE, bool LIN, int BY, int BX, class BLK>
 __device__ __forceinline__ void vanka_sweep_tile(const SweepArgs<R>& a, int gmode, BLK blk) {
-    using TileT = Tile<R, kTile, 2, 1>;
-    constexpr int NC = TileT::NC;     // 19
-    constexpr int ND = kTile + 1;     // deltas for rows/cols [i0-1, i0+16)
+    constexpr int TY = BY - 1, TX = BX - 1;
+    using TileT = Tile<R, TY, TX, 2, 1>;
+    constexpr int NR = TileT::NR, NC = TileT::NC;
     __shared__ TileT t;
-    __shared__ R dl[ND][ND][4];
-    const int i0 = blk.y() * kTile, j0 = blk.x() * kTile;
+    __shared__ R dl[BY][BX][4];
+    const int i0 = blk.y() * TY, j0 = blk.x() * TX;
     const int ny = a.ny, nx = a.nx;
-    stage_tile<R, kTile, 2, 1>(t, i0, j0, ny, nx, a.u, a.v, a.H, a.bed, a.beta, PHI_LIVE ? nullptr : &a.phi);
+    stage_tile<R, TY, TX, 2, 1>(t, i0, j0, ny, nx, a.u, a.v, a.H, a.bed, a.beta, PHI_LIVE ? nullptr : &a.phi);
     __syncthreads();
-    TileView<R, kTile, 2, 1> s{t, i0, j0, ny, nx};
-    for (int k = threadIdx.x; k < NC * NC; k += blockDim.x) {
+    TileView<R, TY, TX, 2, 1> s{t, i0, j0, ny, nx};
+    for (int k = threadIdx.x; k < NR * NC; k += BY * BX) {
         int r = k / NC, c = k % NC;
         int gi = i0 - 2 + r, gj = j0 - 2 + c;
         int ci = clampi(gi, 0, ny - 1), cj = clampi(gj, 0, nx - 1);
@@ -205,74 +205,78 @@ __device__ __forceinline__ void vanka_sweep_tile(const SweepArgs<R>& a, int gmod
     }
     __syncthreads();
 
-    // which cell does this thread solve?
-    int i, j;
-    const int tid = threadIdx.x;
-    if (tid < kTile * kTile) { i = i0 + tid / kTile; j = j0 + tid % kTile; }
-    else if (tid < kTile * kTile + kTile) { i = i0 + (tid - kTile * kTile); j = j0 - 1; }
-    else { i = i0 - 1; j = j0 + (tid - kTile * kTile - kTile); }
+    const int di = threadIdx.x / BX, dj = threadIdx.x % BX;
+    const int i = i0 - 1 + di, j = j0 - 1 + dj;
+    const bool own = di > 0 && dj > 0;
     const bool live = i >= 0 && i < ny && j >= 0 && j < nx;
     R dH = 0, masked = 0;
     R dd[4] = {0, 0, 0, 0};
     if (live) {
-        R x[5] = {s.U(i, j), s.U(i, j + 1), s.V(i, j), s.V(i + 1, j), s.Hc(i, j)};
         R thk;
         if (gmode == kGammaArray) thk = a.gamma.at(i, j);
         else if (gmode == kGammaWChi) thk = a.wH.at(i, j) + a.chi.at(i, j);
         else thk = a.wH.at(i, j) + (-a.chi_c.at(i >> 1, j >> 1) + a.chi.at(i, j));
-        masked = tid < kTile * kTile ? a.mask.at(i, j) : R(0);  // halo cells never write it
-        R comp[5] = {0, 0, 0, 0, 0};
-        R rnorm = 1;
+        masked = own ? a.mask.at(i, j) : R(0);  // halo cells never write it
         int k = 0;
-        const R tol = R(kNewtonTol);
-        while (k < a.newton_steps && rnorm > tol) {
-            R J[25], r[5];
-            local_system<R>(s, a.p, i, j, x, J, r);
-            // forcing is re-read each iteration (L1 hits) to keep registers free
-            r[0] -= ldg(&a.f_u.at(i, j)); r[1] -= ldg(&a.f_u.at(i, j + 1));
-            r[2] -= ldg(&a.f_v.at(i, j)); r[3] -= ldg(&a.f_v.at(i + 1, j));
-            r[4] -= ldg(&a.f_H.at(i, j));
-            J[0] -= a.ssa_damping; J[6] -= a.ssa_damping; J[12] -= a.ssa_damping; J[18] -= a.ssa_damping;
-            J[24] += a.mc_damping;
-            if (j == 0) { pin(J, 0); r[0] = x[0]; }
-            if (j == nx - 1) { pin(J, 1); r[1] = x[1]; }
-            if (i == 0) { pin(J, 2); r[2] = x[2]; }
-            if (i == ny - 1) { pin(J, 3); r[3] = x[3]; }
-            if ((x[4] - a.p.dt * r[4]) <= thk) {
-                masked = R(1);
-                pin(J, 4);
-                r[4] = x[4] - thk;
-            } else {
-                masked = R(0);
-            }
-            // squared norm of the pre-update local residual (vanka.cu:613)
-            rnorm = r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3] + r[4] * r[4];
-            lu5_solve(J, r, r);
+        if constexpr (LIN) {
+            LocalCell<R> cell;
+            cell.load(s, a.p, i, j, ldg(&a.f_u.at(i, j)), ldg(&a.f_u.at(i, j + 1)), ldg(&a.f_v.at(i, j)),
+                      ldg(&a.f_v.at(i + 1, j)), ldg(&a.f_H.at(i, j)));
+            R d[5] = {0, 0, 0, 0, 0};
+            k = cell.solve(a.p, a.ssa_damping, a.mc_damping, a.relax, thk, a.newton_steps, d, masked);
 #pragma unroll
-            for (int q = 0; q < 5; ++q) {  // compensated (Kahan) update, vanka.cu:617-640
-                R y = -a.relax * r[q] - comp[q];
-                R tq = x[q] + y;
-                comp[q] = (tq - x[q]) - y;
-                x[q] = tq;
+            for (int q = 0; q < 4; ++q) dd[q] = R(0.5) * d[q];
+            dH = d[4];
+        } else {
+            R x[5] = {s.U(i, j), s.U(i, j + 1), s.V(i, j), s.V(i + 1, j), s.Hc(i, j)};
+            R comp[5] = {0, 0, 0, 0, 0};
+            R rnorm = 1;
+            const R tol = R(kNewtonTol);
+            while (k < a.newton_steps && rnorm > tol) {
+                R J[25], r[5];
+                local_system<R>(s, a.p, i, j, x, J, r);
+                // forcing is re-read each iteration (L1 hits) to keep registers free
+                r[0] -= ldg(&a.f_u.at(i, j)); r[1] -= ldg(&a.f_u.at(i, j + 1));
+                r[2] -= ldg(&a.f_v.at(i, j)); r[3] -= ldg(&a.f_v.at(i + 1, j));
+                r[4] -= ldg(&a.f_H.at(i, j));
+                J[0] -= a.ssa_damping; J[6] -= a.ssa_damping; J[12] -= a.ssa_damping; J[18] -= a.ssa_damping;
+                J[24] += a.mc_damping;
+                if (j == 0) { pin(J, 0); r[0] = x[0]; }
+                if (j == nx - 1) { pin(J, 1); r[1] = x[1]; }
+                if (i == 0) { pin(J, 2); r[2] = x[2]; }
+                if (i == ny - 1) { pin(J, 3); r[3] = x[3]; }
+                if ((x[4] - a.p.dt * r[4]) <= thk) {
+                    masked = R(1);
+                    pin(J, 4);
+                    r[4] = x[4] - thk;
+                } else {
+                    masked = R(0);
+                }
+                // squared norm of the pre-update local residual (vanka.cu:613)
+                rnorm = r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3] + r[4] * r[4];
+                lu5_solve(J, r, r);
+#pragma unroll
+                for (int q = 0; q < 5; ++q) {  // compensated (Kahan) update, vanka.cu:617-640
+                    R y = -a.relax * r[q] - comp[q];
+                    R tq = x[q] + y;
+                    comp[q] = (tq - x[q]) - y;
+                    x[q] = tq;
+                }
+                x[4] = fmax(x[4], thk);
+                ++k;
             }
-            x[4] = fmax(x[4], thk);
-            ++k;
+            dd[0] = R(0.5) * (x[0] - s.U(i, j));
+            dd[1] = R(0.5) * (x[1] - s.U(i, j + 1));
+            dd[2] = R(0.5) * (x[2] - s.V(i, j));
+            dd[3] = R(0.5) * (x[3] - s.V(i + 1, j));
+            dH = x[4] - s.Hc(i, j);
         }
-        if (a.iters && tid < kTile * kTile) a.iters[size_t(i) * a.phi.pitch + j] = k;
-        dd[0] = R(0.5) * (x[0] - s.U(i, j));
-        dd[1] = R(0.5) * (x[1] - s.U(i, j + 1));
-        dd[2] = R(0.5) * (x[2] - s.V(i, j));
-        dd[3] = R(0.5) * (x[3] - s.V(i + 1, j));
-        dH = x[4] - s.Hc(i, j);
+        if (a.iters && own) a.iters[size_t(i) * a.phi.pitch + j] = k;
     }
-    {
-        const int di = i - (i0 - 1), dj = j - (j0 - 1);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) dl[di][dj][q] = dd[q];
-    }
+    for (int q = 0; q < 4; ++q) dl[di][dj][q] = dd[q];
     __syncthreads();
-    if (tid < kTile * kTile && live) {
-        const int di = i - (i0 - 1), dj = j - (j0 - 1);
+    if (own && live) {
         const R w = a.omega;
         // left face: right half-correction of cell (i, j-1) + left of (i, j)
         R du = (j > 0 ? dl[di][dj - 1][1] : R(0)) + dl[di][dj][0];
@@ -287,9 +291,17 @@ __device__ __forceinline__ void vanka_sweep_tile(const SweepArgs<R>& a, int gmod
     }
 }
 
-template <class R, int GMODE, bool PHI_LIVE, int MINB>
-__global__ void __launch_bounds__(kSweepThreads, MINB) k_vanka_sweep(SweepArgs<R> a) {
-    vanka_sweep_tile<R, PHI_LIVE>(a, GMODE, SoloBlock{});
+// A compiled form of the sweep: local iteration, block shape and the resident
+// blocks per SM its registers are fitted to.
+template <bool LIN, int BY, int BX, int MINB>
+struct SweepForm {
+    static constexpr bool kLinear = LIN;
+    static constexpr int kBY = BY, kBX = BX, kThreads = BY * BX, kMinBlocks = MINB;
+};
+
+template <class R, bool PHI_LIVE, class Form>
+__global__ void __launch_bounds__(Form::kThreads, Form::kMinBlocks) k_vanka_sweep(SweepArgs<R> a) {
+    vanka_sweep_tile<R, PHI_LIVE, Form::kLinear, Form::kBY, Form::kBX>(a, a.gmode, SoloBlock{});
 }
 
 }  // namespace glide

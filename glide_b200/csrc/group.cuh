@@ -223,13 +223,13 @@ struct OpMaps<Op, std::void_t<decltype(Op::kMaps)>> {
 };
 
 // Register budgets: the per-hierarchy kernels' resident blocks per SM.
-template <class R, bool PHI_LIVE, int MINB>
+template <class R, bool PHI_LIVE, class Form>
 struct GSweep {
-    static constexpr int kMinBlocks = MINB;
+    static constexpr int kMinBlocks = Form::kMinBlocks;
     using Args = SweepArgs<R>;
-    static constexpr int kThreads = kSweepThreads;
+    static constexpr int kThreads = Form::kThreads;
     static __device__ __forceinline__ void run(const Args& a, const unsigned char*, GroupBlock b) {
-        vanka_sweep_tile<R, PHI_LIVE>(a, a.gmode, b);
+        vanka_sweep_tile<R, PHI_LIVE, Form::kLinear, Form::kBY, Form::kBX>(a, a.gmode, b);
     }
 };
 template <class R>

@@ -160,7 +160,7 @@ struct SolverBase {
     int quirks = 1;
     int use_graphs = 1;
     unsigned version = 1;
-    // Vanka sweep register budget: resident blocks per SM (1 or 2)
+    // general Vanka sweep's register budget: resident blocks per SM (1 or 2)
     int sweep_blocks_per_sm = 2;
     // forward solve: 0 = FASCD V-cycles only (the reference's method);
     // 1 = FASCD until rel. residual <= newton_switch, then Newton steps whose
@@ -180,6 +180,25 @@ struct RecOp {
     double bytes;
     std::vector<unsigned char> maps;  // the staging maps of a stencil launch (BoxMaps)
 };
+
+// The forms of the Vanka sweep a launch picks from.  The linear-sliding form
+// runs 8 x 16 blocks (7 x 15 owned cells): four warps fill the four register
+// files evenly, so binary64 fits 168 registers at 3 blocks per SM without
+// spilling to speak of, and small levels spread over many SMs.  Measured, ms
+// per 3-V-cycle step in binary64 on 512^2 / 64^2: 8 x 16 at 3 blocks 26.7 /
+// 10.5, 12 x 16 at 2 blocks 27.4 / 13.5, 24 x 16 at 1 block 30.9 / 16.0,
+// 8 x 16 at 4 blocks 29.3 / 13.1.  In binary32 (600 x 424, 2 V-cycles) 5
+// blocks per SM run 9.36, 3 or 4 blocks 9.74.
+enum SweepFormId { S_GENERAL_1, S_GENERAL_2, S_LINEAR };
+template <class R, class F>
+static void with_sweep_form(int form, F&& f) {
+    switch (form) {
+        case S_GENERAL_1: f(SweepForm<false, 16, 16, 1>{}); break;
+        case S_GENERAL_2: f(SweepForm<false, 16, 16, 2>{}); break;
+        case S_LINEAR: f(SweepForm<true, 8, 16, sizeof(R) == 8 ? 3 : 5>{}); break;
+        default: fail(GLIDE_ERR_STATE, "unknown sweep form");
+    }
+}
 
 template <class R>
 struct Solver;
@@ -553,7 +572,7 @@ struct Solver : SolverBase {
         a.relax = quirks ? R(0.5) : R(c.relaxation);
         a.newton_steps = c.newton_steps;
         a.ny = v.ny; a.nx = v.nx;
-        dim3 g(v.blocks_x(), v.blocks_y());
+        a.gmode = gmode;
         for (int k = 0; k < n; ++k) {
             const bool in_alt = (start_alt ^ (k & 1)) != 0;
             const int U0 = GLIDE_U, V0 = GLIDE_V, H0 = GLIDE_H, U1 = F_U_ALT, V1 = F_V_ALT, H1 = F_H_ALT;
@@ -571,31 +590,29 @@ struct Solver : SolverBase {
                     counted("grounded", lb(l, 4));
                 }
             }
-            launch_sweep(a, gmode, phi_live, g, s, lb(l, 15));
+            launch_sweep(a, phi_live, s, lb(l, 15));
         }
-    }
-
-    template <int MINB>
-    void launch_sweep_occ(const SweepArgs<R>& a, int gmode, bool phi_live, dim3 g, cudaStream_t s) {
-#define GLIDE_SWEEP(GM, PL) k_vanka_sweep<R, GM, PL, MINB><<<g, kSweepThreads, 0, s>>>(a)
-        if (gmode == kGammaArray) { if (phi_live) GLIDE_SWEEP(kGammaArray, true); else GLIDE_SWEEP(kGammaArray, false); }
-        else if (gmode == kGammaWChi) { if (phi_live) GLIDE_SWEEP(kGammaWChi, true); else GLIDE_SWEEP(kGammaWChi, false); }
-        else { if (phi_live) GLIDE_SWEEP(kGammaWPhi, true); else GLIDE_SWEEP(kGammaWPhi, false); }
-#undef GLIDE_SWEEP
     }
 
     // one fused sweep: u, v, H, f_u, f_v, f_H, bed, B, beta, gamma, phi read;
     // u, v, H, mask written (15 N s)
-    void launch_sweep(const SweepArgs<R>& a, int gmode, bool phi_live, dim3 g, cudaStream_t s, double bytes) {
-        if (rec) {
-            SweepArgs<R> ga = a;
-            ga.gmode = gmode;
-            record(G_SWEEP, (phi_live ? 1 : 0) | (sweep_blocks_per_sm >= 2 ? 2 : 0), g, ga, bytes);
-            return;
-        }
-        if (sweep_blocks_per_sm >= 2) launch_sweep_occ<2>(a, gmode, phi_live, g, s);
-        else launch_sweep_occ<1>(a, gmode, phi_live, g, s);
+    template <class Form>
+    void launch_sweep_form(const SweepArgs<R>& a, bool phi_live, int variant, cudaStream_t s, double bytes) {
+        const dim3 g((a.nx + Form::kBX - 2) / (Form::kBX - 1), (a.ny + Form::kBY - 2) / (Form::kBY - 1));
+        if (record(G_SWEEP, variant, g, a, bytes)) return;
+        if (phi_live) k_vanka_sweep<R, true, Form><<<g, Form::kThreads, 0, s>>>(a);
+        else k_vanka_sweep<R, false, Form><<<g, Form::kThreads, 0, s>>>(a);
         counted("vanka_sweep", bytes);
+    }
+
+    void launch_sweep(const SweepArgs<R>& a, bool phi_live, cudaStream_t s, double bytes) {
+        // the linear-sliding form divides by diagonals of at least this sum
+        // (local_cell.cuh); any other exponent or damping takes the general one
+        const bool linear = a.p.m == R(1) && a.ssa_damping + a.p.water_drag > R(0);
+        const int form = linear ? S_LINEAR : (sweep_blocks_per_sm >= 2 ? S_GENERAL_2 : S_GENERAL_1);
+        with_sweep_form<R>(form, [&](auto f) {
+            launch_sweep_form<decltype(f)>(a, phi_live, (phi_live ? 1 : 0) | 2 * form, s, bytes);
+        });
     }
 
     // Restrictions of several fields of level l in one launch; each job is
@@ -1562,9 +1579,14 @@ struct GroupRun : GroupBase {
             case G_RESIDUAL: return issue_op<GResidual<R>>(L, s);
             case G_VJP: return issue_op<GVjp<R>>(L, s);
             case G_JVP: return issue_op<GJvp<R>>(L, s);
-            case G_SWEEP:
-                if (v & 2) return (v & 1) ? issue_op<GSweep<R, true, 2>>(L, s) : issue_op<GSweep<R, false, 2>>(L, s);
-                return (v & 1) ? issue_op<GSweep<R, true, 1>>(L, s) : issue_op<GSweep<R, false, 1>>(L, s);
+            case G_SWEEP: {
+                long long issued = 0;
+                with_sweep_form<R>(v >> 1, [&](auto f) {
+                    issued = (v & 1) ? issue_op<GSweep<R, true, decltype(f)>>(L, s)
+                                     : issue_op<GSweep<R, false, decltype(f)>>(L, s);
+                });
+                return issued;
+            }
             case G_BLOCK_FACTOR:
                 return v ? issue_op<GBlockFactor<R, true>>(L, s) : issue_op<GBlockFactor<R, false>>(L, s);
             case G_BLOCK_SWEEP:
