@@ -25,7 +25,7 @@
 #include "glide_b200.h"
 #include "adjoint_kernels.cuh"
 #include "forward_kernels.cuh"
-#include "tangent_kernels.cuh"
+#include "strip.cuh"
 #include "transfer_kernels.cuh"
 
 namespace glide {
@@ -33,14 +33,8 @@ namespace glide {
 // Launch kinds a hierarchy records for grouped execution.
 enum GroupOpKind {
     G_SNAPSHOT, G_RESTRICT, G_RESTRICT_BATCH, G_CORRECT_BATCH, G_GROUNDED, G_COPY, G_SET_RHS, G_SWEEP,
-    G_RESIDUAL, G_NORMS, G_VJP, G_BLOCK_FACTOR, G_BLOCK_SWEEP, G_GRADIENTS, G_FILL, G_JVP, G_TANGENT_RHS,
-    G_NEWTON_UPDATE, G_KINDS
-};
-
-template <class R>
-struct JvpOpArgs {
-    VjpArgs<R> a;
-    int mode;
+    G_RESIDUAL, G_NORMS, G_LINEAR, G_SMOOTH, G_BLOCK_FACTOR, G_GRADIENTS, G_FILL, G_TANGENT_RHS, G_NEWTON_UPDATE,
+    G_KINDS
 };
 
 struct NormsArgs {
@@ -242,24 +236,13 @@ struct GResidual {
         residual_tile<R>(a, item_maps<7>(mp), b);
     }
 };
-template <class R>
-struct GVjp {
-    static constexpr int kMaps = 9;
-    static constexpr int kMinBlocks = sizeof(R) == 8 ? 2 : 3;
-    using Args = VjpArgs<R>;
-    static constexpr int kThreads = kTileA * kTileA;
-    static __device__ __forceinline__ void run(const Args& a, const unsigned char* mp, GroupBlock b) {
-        vjp_tile<R>(a, item_maps<9>(mp), b);
-    }
-};
-template <class R>
-struct GJvp {
-    static constexpr int kMaps = JvpTile<R>::NB;
-    static constexpr int kMinBlocks = sizeof(R) == 8 ? 3 : 6;
-    using Args = JvpOpArgs<R>;
-    static constexpr int kThreads = kTileA * kTileA;
-    static __device__ __forceinline__ void run(const Args& a, const unsigned char* mp, GroupBlock b) {
-        jvp_tile<R>(a.a, a.mode, item_maps<JvpTile<R>::NB>(mp), b);
+template <class R, bool TR, bool SMOOTH>
+struct GLinear {
+    static constexpr int kMinBlocks = StripBlocks<R, SMOOTH>::n;
+    using Args = StripArgs<R>;
+    static constexpr int kThreads = 32 * kStripWarps;
+    static __device__ __forceinline__ void run(const Args& a, const unsigned char*, GroupBlock b) {
+        linear_strip<R, TR, SMOOTH>(a, b);
     }
 };
 template <class R, bool TR>
@@ -272,16 +255,6 @@ struct GBlockFactor {
         block_factor_tile<R, TR>(a, item_maps<7>(mp), b);
     }
 };
-template <class R, bool TR>
-struct GBlockSweep {
-    static constexpr int kMinBlocks = sizeof(R) == 8 ? 4 : 5;
-    using Args = BlockArgs<R>;
-    static constexpr int kThreads = kSweepThreads;
-    static __device__ __forceinline__ void run(const Args& a, const unsigned char*, GroupBlock b) {
-        block_sweep_tile<R, TR>(a, b);
-    }
-};
-
 // The item holding tile t: the last item whose range starts at or before t.
 template <class A, int N>
 __device__ __forceinline__ int group_item_of(const GroupParams<A, N>& P, int t) {

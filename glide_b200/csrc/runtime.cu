@@ -23,7 +23,7 @@
 #include "glide_b200.h"
 #include "forward_kernels.cuh"
 #include "adjoint_kernels.cuh"
-#include "tangent_kernels.cuh"
+#include "strip.cuh"
 #include "transfer_kernels.cuh"
 #include "group.cuh"
 
@@ -70,6 +70,8 @@ enum InternalField {
     // tangent (Newton correction) system: correction, right-hand side,
     // residual and the coarse-level snapshot of the correction
     F_E_U, F_E_V, F_E_H, F_TF_U, F_TF_V, F_TF_H, F_TR_U, F_TR_V, F_TR_H, F_TW_U, F_TW_V, F_TW_H,
+    // second buffer of the linear smoother's unknowns
+    F_XA_U, F_XA_V, F_XA_H,
     // state before a Newton step, restored when the step is rejected
     F_BK_U, F_BK_V, F_BK_H, F_BK_MASK,
     F_COUNT
@@ -82,12 +84,12 @@ static Kind field_kind(int f) {
         case GLIDE_U: case GLIDE_F_U: case GLIDE_R_U: case GLIDE_LAMBDA_U: case GLIDE_ADJ_F_U:
         case GLIDE_ADJ_R_U: case GLIDE_VJP_U: case GLIDE_FOP_U: case F_U_ALT: case F_W_U: case F_WL_U:
         case F_E_U: case F_TF_U: case F_TR_U: case F_TW_U: case GLIDE_VAR_U: case GLIDE_JVP_U:
-        case F_BK_U:
+        case F_BK_U: case F_XA_U:
             return KU;
         case GLIDE_V: case GLIDE_F_V: case GLIDE_R_V: case GLIDE_LAMBDA_V: case GLIDE_ADJ_F_V:
         case GLIDE_ADJ_R_V: case GLIDE_VJP_V: case GLIDE_FOP_V: case F_V_ALT: case F_W_V: case F_WL_V:
         case F_E_V: case F_TF_V: case F_TR_V: case F_TW_V: case GLIDE_VAR_V: case GLIDE_JVP_V:
-        case F_BK_V:
+        case F_BK_V: case F_XA_V:
             return KV;
         default:
             return KC;
@@ -181,21 +183,24 @@ struct RecOp {
     std::vector<unsigned char> maps;  // the staging maps of a stencil launch (BoxMaps)
 };
 
-// The forms of the Vanka sweep a launch picks from.  The linear-sliding form
-// runs 8 x 16 blocks (7 x 15 owned cells): four warps fill the four register
-// files evenly, so binary64 fits 168 registers at 3 blocks per SM without
-// spilling to speak of, and small levels spread over many SMs.  Measured, ms
-// per 3-V-cycle step in binary64 on 512^2 / 64^2: 8 x 16 at 3 blocks 26.7 /
-// 10.5, 12 x 16 at 2 blocks 27.4 / 13.5, 24 x 16 at 1 block 30.9 / 16.0,
-// 8 x 16 at 4 blocks 29.3 / 13.1.  In binary32 (600 x 424, 2 V-cycles) 5
-// blocks per SM run 9.36, 3 or 4 blocks 9.74.
+// The forms of the Vanka sweep a launch picks from: the general one at one of
+// two register budgets, or the linear-sliding one.
+//
+// Blocks of whole groups of four warps fill the four register files evenly
+// (288-thread blocks left a quarter of them idle).  Binary64, general: 8 x 16
+// threads (7 x 15 owned cells) at 3 per SM run a 3-V-cycle step of 512^2 / 64^2
+// in 53.2 / 27.8 ms, 16 x 16 at 2 per SM 54.1 / 34.8, 8 x 16 at 4 per SM 54.7 /
+// 32.3, 8 x 8 at 5 per SM 58.0 / 29.4; 288-thread blocks took 56.5 / 31.1.
+// Binary32, linear (600 x 424, 2 V-cycles): 8 x 16 at 5 per SM 9.36 ms, at 3 or
+// 4 per SM 9.74.
 enum SweepFormId { S_GENERAL_1, S_GENERAL_2, S_LINEAR };
 template <class R, class F>
 static void with_sweep_form(int form, F&& f) {
+    constexpr bool wide = sizeof(R) == 8;
     switch (form) {
-        case S_GENERAL_1: f(SweepForm<false, 16, 16, 1>{}); break;
-        case S_GENERAL_2: f(SweepForm<false, 16, 16, 2>{}); break;
-        case S_LINEAR: f(SweepForm<true, 8, 16, sizeof(R) == 8 ? 3 : 5>{}); break;
+        case S_GENERAL_1: f(SweepForm<false, wide ? 8 : 16, 16, wide ? 2 : 1>{}); break;
+        case S_GENERAL_2: f(SweepForm<false, wide ? 8 : 16, 16, wide ? 3 : 2>{}); break;
+        case S_LINEAR: f(SweepForm<!wide, 8, 16, wide ? 3 : 5>{}); break;
         default: fail(GLIDE_ERR_STATE, "unknown sweep form");
     }
 }
@@ -215,6 +220,11 @@ struct Level {
     int blocks_y() const { return (ny + kTile - 1) / kTile; }
 };
 
+template <bool SMOOTH>
+static int strip_cols(int nx) {
+    return (nx + StripShape<SMOOTH>::kCols) / StripShape<SMOOTH>::kCols;  // columns 0 .. nx
+}
+
 template <class R>
 struct Solver : SolverBase {
     std::vector<Level<R>> lv;
@@ -224,10 +234,8 @@ struct Solver : SolverBase {
     double* norms_host = nullptr;
     int* err_dev = nullptr;  // kStage* bits set by a staging block (its wait gave up, or its maps failed their check)
     // TMA tensor maps of every (level, field), encoded on first use
-    // slot per box height (kTmaHeights)
-    static constexpr int kTmaHeights[3] = {kBoxH, 22, 24};
-    std::vector<CUtensorMap> tmaps[3];
-    std::vector<unsigned char> tmap_done[3];
+    std::vector<CUtensorMap> tmaps;
+    std::vector<unsigned char> tmap_done;
     bool use_tma = true;
     int tma_wait_polls = kTmaWaitPolls;  // 0 under GLIDE_TUNE_TMA_GIVE_UP
     // one captured V-cycle per cycle kind (0 FAS, 1 adjoint, 2 mixed FAS,
@@ -329,7 +337,9 @@ struct Solver : SolverBase {
                 bytes += (size_t(rows) * pitch * sizeof(R) + align - 1) / align * align;
             }
         }
-        const int nblk = lv[0].blocks_x() * lv[0].blocks_y();
+        // norm partials: one slot per block of a stencil pass or of a march
+        const int nblk = std::max(lv[0].blocks_x() * lv[0].blocks_y(),
+                                  strip_cols<false>(lv[0].nx) * ((lv[0].ny + kStripWarps - 1) / kStripWarps));
         size_t partial_off = bytes;
         bytes += (size_t(nblk) * 3 * sizeof(double) + align - 1) / align * align;
         size_t norms_off = bytes;
@@ -506,43 +516,40 @@ struct Solver : SolverBase {
     }
 
     // TMA staging needs a level at least one box wide and high
-    bool tma_level(int l, int bh = kBoxH) const { return use_tma && lv[l].nx >= kBoxW && lv[l].ny >= bh; }
+    bool tma_level(int l) const { return use_tma && lv[l].nx >= kBoxW && lv[l].ny >= kBoxH; }
 
-    const CUtensorMap& tmap(int l, int f, int bh = kBoxH) {
-        int w = 0;
-        while (w < 3 && kTmaHeights[w] != bh) ++w;
-        if (w == 3) fail(GLIDE_ERR_STATE, "no tensor-map slot for this box height");
-        if (tmaps[w].empty()) {
-            tmaps[w].resize(size_t(n_levels) * F_COUNT);
-            tmap_done[w].assign(size_t(n_levels) * F_COUNT, 0);
+    const CUtensorMap& tmap(int l, int f) {
+        if (tmaps.empty()) {
+            tmaps.resize(size_t(n_levels) * F_COUNT);
+            tmap_done.assign(size_t(n_levels) * F_COUNT, 0);
         }
         const size_t k = size_t(l) * F_COUNT + f;
-        if (!tmap_done[w][k]) {
+        if (!tmap_done[k]) {
             PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
             if (!enc) fail(GLIDE_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
             const Arr<R>& a = lv[l].a[f];
             const cuuint64_t dims[2] = {cuuint64_t(a.cols), cuuint64_t(a.rows)};
             const cuuint64_t strides[1] = {cuuint64_t(a.pitch) * sizeof(R)};
-            const cuuint32_t box[2] = {cuuint32_t(kBoxW), cuuint32_t(bh)};
+            const cuuint32_t box[2] = {cuuint32_t(kBoxW), cuuint32_t(kBoxH)};
             const cuuint32_t estr[2] = {1, 1};
-            const CUresult r = enc(&tmaps[w][k], sizeof(R) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64
+            const CUresult r = enc(&tmaps[k], sizeof(R) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64
                                                                   : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
                                    2, a.p, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             if (r != CUDA_SUCCESS) fail(GLIDE_ERR_CUDA, "cuTensorMapEncodeTiled failed");
-            tmap_done[w][k] = 1;
+            tmap_done[k] = 1;
         }
-        return tmaps[w][k];
+        return tmaps[k];
     }
 
     template <int N>
-    BoxMaps<N> box_maps(int l, const int (&fields)[N], int bh = kBoxH) {
+    BoxMaps<N> box_maps(int l, const int (&fields)[N]) {
         BoxMaps<N> m;
-        m.use = tma_level(l, bh) ? 1 : 0;
+        m.use = tma_level(l) ? 1 : 0;
         m.wait_polls = tma_wait_polls;
         if (m.use)
-            for (int q = 0; q < N; ++q) m.m[q] = tmap(l, fields[q], bh);
+            for (int q = 0; q < N; ++q) m.m[q] = tmap(l, fields[q]);
         return m;
     }
 
@@ -606,9 +613,13 @@ struct Solver : SolverBase {
     }
 
     void launch_sweep(const SweepArgs<R>& a, bool phi_live, cudaStream_t s, double bytes) {
-        // the linear-sliding form divides by diagonals of at least this sum
-        // (local_cell.cuh); any other exponent or damping takes the general one
-        const bool linear = a.p.m == R(1) && a.ssa_damping + a.p.water_drag > R(0);
+        // The linear-sliding form reorders the local system's sums and divides
+        // by diagonals of at least damping + drag (local_cell.cuh).  Binary64
+        // keeps the general form: the local iteration stops on a threshold, a
+        // reordered sum flips a cell's count there now and then (measured in 2
+        // of 26 adjoint runs at 512^2, up to 4e-9 in the gradients), and
+        // binary64 promises the reference's iterates.
+        const bool linear = sizeof(R) == 4 && a.p.m == R(1) && a.ssa_damping + a.p.water_drag > R(0);
         const int form = linear ? S_LINEAR : (sweep_blocks_per_sm >= 2 ? S_GENERAL_2 : S_GENERAL_1);
         with_sweep_form<R>(form, [&](auto f) {
             launch_sweep_form<decltype(f)>(a, phi_live, (phi_live ? 1 : 0) | 2 * form, s, bytes);
@@ -1017,47 +1028,55 @@ struct Solver : SolverBase {
                 {F_TW_U, F_TW_V, F_TW_H}, false, 2};
     }
 
-    // out = Op(x) [- f] [- sub], Op = J^T (vjp) or J (jvp) at the level's state
-    // jvp_flags (the JVP only): GLIDE_USE_MASK and GLIDE_FREEZE_CALVING as in
-    // glide_jvp; the solver's own tangent operator keeps the mask and calving.
-    void lin_op(int l, double dt, const Lin& L, const int* out, const int* sub, bool use_forcing, bool norms,
-                bool ref_rows, cudaStream_t s, int jvp_flags = GLIDE_USE_MASK) {
+    // The linear operator's fields at level l's state: x in, out = Op(x) [- f]
+    // [- sub], Op = J^T or J.  jvp_flags (J only): GLIDE_USE_MASK and
+    // GLIDE_FREEZE_CALVING as in glide_jvp; the solver's own tangent operator
+    // keeps the mask and calving.
+    StripArgs<R> strip_args(int l, double dt, const Lin& L, const int* out, const int* sub, bool use_forcing,
+                            bool norms, bool ref_rows, int jvp_flags) {
         Level<R>& v = lv[l];
-        VjpArgs<R> a;
+        StripArgs<R> q{};
+        VjpArgs<R>& a = q.a;
         a.u = v.a[GLIDE_U]; a.v = v.a[GLIDE_V]; a.H = v.a[GLIDE_H];
         a.phi = v.a[GLIDE_PHI]; a.mask = v.a[GLIDE_MASK]; a.bed = v.a[GLIDE_BED]; a.B = v.a[GLIDE_B];
         a.beta = v.a[GLIDE_BETA];
         a.lu = v.a[L.x[0]]; a.lv = v.a[L.x[1]]; a.lH = v.a[L.x[2]];
         a.f_u = v.a[L.f[0]]; a.f_v = v.a[L.f[1]]; a.f_H = v.a[L.f[2]];
-        a.o_u = v.a[out[0]]; a.o_v = v.a[out[1]]; a.o_H = v.a[out[2]];
+        if (out) { a.o_u = v.a[out[0]]; a.o_v = v.a[out[1]]; a.o_H = v.a[out[2]]; }
         if (sub) { a.s_u = v.a[sub[0]]; a.s_v = v.a[sub[1]]; a.s_H = v.a[sub[2]]; }
         a.partial = norms ? partial : nullptr;
-        a.err = err_dev;
         a.p = physr(l, dt, !L.tr && (jvp_flags & GLIDE_FREEZE_CALVING));
         a.ny = v.ny; a.nx = v.nx; a.use_forcing = use_forcing;
-        dim3 g((a.nx + kTileA - 1) / kTileA, (a.ny + kTileA - 1) / kTileA);
+        q.mode = (ref_rows ? 1 : 0) | ((jvp_flags & GLIDE_USE_MASK) ? 0 : 2);
+        return q;
+    }
+
+    // Rows of a chunk: every chunk feeds two or three rows more than it owns,
+    // so as many as leave the GPU enough warps (binary32 16 to 20 resident per
+    // SM and two waves of them, binary64 8 to 12 and one), between 2 and 32.
+    // Measured: 512^2 binary64 gradient 9.9 ms with 2400 warps aimed at, 11.1
+    // with 4800; 2048^2 mixed gradient 33.2 with 4800, 36.6 with 2400 and up to
+    // 64 rows; one row a chunk loses 10 % on eight grouped 192^2 members.
+    template <bool SMOOTH>
+    dim3 strip_grid(StripArgs<R>& q) const {
+        constexpr int target = sizeof(R) == 8 ? 2400 : 4800;
+        const int cols = strip_cols<SMOOTH>(q.a.nx);
+        q.rows = std::min(32, std::max(2, int((long long)q.a.ny * cols / target)));
+        const int per_block = q.rows * kStripWarps;
+        return dim3(cols, (q.a.ny + per_block - 1) / per_block);
+    }
+
+    void lin_op(int l, double dt, const Lin& L, const int* out, const int* sub, bool use_forcing, bool norms,
+                bool ref_rows, cudaStream_t s, int jvp_flags = GLIDE_USE_MASK) {
+        StripArgs<R> q = strip_args(l, dt, L, out, sub, use_forcing, norms, ref_rows, jvp_flags);
+        const dim3 g = strip_grid<false>(q);
         // u, v, H, phi, mask, bed, beta, B and the three unknowns read, the
         // forcing and the subtrahend when given, three rows written
-        const double lin_bytes = lb(l, 11 + (use_forcing ? 3 : 0) + (sub ? 3 : 0) + 3);
-        if (L.tr) {
-            const int fl[AdjTile<R>::NB] = {GLIDE_U, GLIDE_V, GLIDE_H, GLIDE_PHI, GLIDE_BED, GLIDE_BETA,
-                                            GLIDE_B, L.x[0], L.x[1]};
-            if (record(G_VJP, 0, g, a, lin_bytes)) {
-                attach_maps(box_maps(l, fl, AdjTile<R>::BH));
-            } else {
-                k_vjp<R><<<g, kTileA * kTileA, 0, s>>>(a, box_maps(l, fl, AdjTile<R>::BH));
-                counted("vjp", lin_bytes);
-            }
-        } else {
-            const int fl[JvpTile<R>::NB] = {GLIDE_U, GLIDE_V, L.x[0], L.x[1], GLIDE_H, GLIDE_PHI, GLIDE_BED,
-                                            GLIDE_BETA, GLIDE_B, L.x[2]};
-            const int mode = (ref_rows ? 1 : 0) | ((jvp_flags & GLIDE_USE_MASK) ? 0 : 2);
-            if (record(G_JVP, 0, g, JvpOpArgs<R>{a, mode}, lin_bytes)) {
-                attach_maps(box_maps(l, fl));
-            } else {
-                k_jvp<R><<<g, kTileA * kTileA, 0, s>>>(a, mode, box_maps(l, fl));
-                counted("jvp", lin_bytes);
-            }
+        const double bytes = lb(l, 11 + (use_forcing ? 3 : 0) + (sub ? 3 : 0) + 3);
+        if (!record(G_LINEAR, L.tr ? 1 : 0, g, q, bytes)) {
+            if (L.tr) k_linear_strip<R, true, false><<<g, 32 * kStripWarps, 0, s>>>(q);
+            else k_linear_strip<R, false, false><<<g, 32 * kStripWarps, 0, s>>>(q);
+            counted(L.tr ? "vjp" : "jvp", bytes);
         }
         if (norms) finish_norms(int(g.x * g.y), s);
     }
@@ -1119,18 +1138,50 @@ struct Solver : SolverBase {
         counted("block_factor", bytes);
     }
 
-    // n linear smoother sweeps (residual, then block solve and update); the
-    // factors are refreshed first unless the caller just did
+    // n linear smoother sweeps (residual, block solve and update in one pass,
+    // alternating between the unknowns' home and second buffers, ending at
+    // home); the factors are refreshed first unless the caller just did
     void lin_sweeps(int l, double dt, int n, const Lin& L, cudaStream_t s, bool factor = true) {
         if (n <= 0) return;
         if (factor) block_factor(l, dt, L, s);
-        BlockArgs<R> a = block_args(l, dt, L);
-        dim3 g(lv[l].blocks_x(), lv[l].blocks_y());
+        if (blk.empty()) fail(GLIDE_ERR_STATE, "block factor buffers not allocated");
+        Level<R>& v = lv[l];
+        const int alt[3] = {F_XA_U, F_XA_V, F_XA_H};
+        StripArgs<R> q = strip_args(l, dt, L, nullptr, nullptr, true, false, false, GLIDE_USE_MASK);
+        q.fac = blk[l];
+        q.plane = size_t(v.ny) * v.pc;
+        q.omega = R(v.vk[L.cfg].omega);
+        const dim3 g = strip_grid<true>(q);
+        const int start_alt = n & 1;
+        if (start_alt)
+            for (int k = 0; k < 3; ++k) copy(v.a[alt[k]], v.a[L.x[k]], s);
+        // u, v, H, phi, mask, bed, beta, B, the unknowns and the forcing read, the
+        // factors read, the unknowns written
+        const double bytes = lb(l, 8 + 3 + 3 + 3) + factor_bytes(l, L.tr);
         for (int k = 0; k < n; ++k) {
-            lin_residual(l, dt, L, false, s);
-            block_sweep(l, a, L.tr, g, s);
+            const bool in_alt = (start_alt ^ (k & 1)) != 0;
+            const int* in = in_alt ? alt : L.x;
+            const int* out = in_alt ? L.x : alt;
+            q.a.lu = v.a[in[0]]; q.a.lv = v.a[in[1]]; q.a.lH = v.a[in[2]];
+            q.xu = v.a[out[0]]; q.xv = v.a[out[1]]; q.xH = v.a[out[2]];
+            if (keep_residual && k == n - 1) {
+                q.a.o_u = v.a[L.r[0]]; q.a.o_v = v.a[L.r[1]]; q.a.o_H = v.a[L.r[2]];
+            }
+            if (record(G_SMOOTH, L.tr ? 1 : 0, g, q, bytes)) continue;
+            if (L.tr) k_linear_strip<R, true, true><<<g, 32 * kStripWarps, 0, s>>>(q);
+            else k_linear_strip<R, false, true><<<g, 32 * kStripWarps, 0, s>>>(q);
+            counted("linear_sweep", bytes);
         }
     }
+
+    // store the residual each group's last sweep starts from (the operator
+    // calls' contract; the solvers recompute theirs)
+    bool keep_residual = false;
+    struct KeepResidual {
+        Solver& s;
+        explicit KeepResidual(Solver& x) : s(x) { s.keep_residual = true; }
+        ~KeepResidual() { s.keep_residual = false; }
+    };
 
     // the 25 factor planes of level l
     double factor_bytes(int l, bool tr) const {
@@ -1142,7 +1193,7 @@ struct Solver : SolverBase {
     // 25 factors, r, x read; x written
     void block_sweep(int l, const BlockArgs<R>& a, bool tr, dim3 g, cudaStream_t s) {
         const double bytes = lb(l, 9) + factor_bytes(l, tr);
-        if (record(G_BLOCK_SWEEP, tr ? 1 : 0, g, a, bytes)) return;
+        not_recordable("a block sweep alone");
         if (tr) k_block_sweep<R, true><<<g, kSweepThreads, 0, s>>>(a);
         else k_block_sweep<R, false><<<g, kSweepThreads, 0, s>>>(a);
         counted("linear_sweep", bytes);
@@ -1392,8 +1443,6 @@ struct GroupRun : GroupBase {
     static size_t maps_bytes(int op) {
         switch (op) {
             case G_RESIDUAL: return sizeof(BoxMaps<OpMaps<GResidual<R>>::n>);
-            case G_VJP: return sizeof(BoxMaps<OpMaps<GVjp<R>>::n>);
-            case G_JVP: return sizeof(BoxMaps<OpMaps<GJvp<R>>::n>);
             case G_BLOCK_FACTOR: return sizeof(BoxMaps<OpMaps<GBlockFactor<R, false>>::n>);
             default: return 0;
         }
@@ -1410,8 +1459,6 @@ struct GroupRun : GroupBase {
     static void untag(int op, unsigned char* p) {
         switch (op) {
             case G_RESIDUAL: return untag<OpMaps<GResidual<R>>::n>(p);
-            case G_VJP: return untag<OpMaps<GVjp<R>>::n>(p);
-            case G_JVP: return untag<OpMaps<GJvp<R>>::n>(p);
             case G_BLOCK_FACTOR: return untag<OpMaps<GBlockFactor<R, false>>::n>(p);
             default: return;
         }
@@ -1577,8 +1624,10 @@ struct GroupRun : GroupBase {
             case G_GRADIENTS: return issue_op<GGradients<R>>(L, s);
             case G_NORMS: return issue_op<GNorms>(L, s);
             case G_RESIDUAL: return issue_op<GResidual<R>>(L, s);
-            case G_VJP: return issue_op<GVjp<R>>(L, s);
-            case G_JVP: return issue_op<GJvp<R>>(L, s);
+            case G_LINEAR:
+                return v ? issue_op<GLinear<R, true, false>>(L, s) : issue_op<GLinear<R, false, false>>(L, s);
+            case G_SMOOTH:
+                return v ? issue_op<GLinear<R, true, true>>(L, s) : issue_op<GLinear<R, false, true>>(L, s);
             case G_SWEEP: {
                 long long issued = 0;
                 with_sweep_form<R>(v >> 1, [&](auto f) {
@@ -1589,8 +1638,6 @@ struct GroupRun : GroupBase {
             }
             case G_BLOCK_FACTOR:
                 return v ? issue_op<GBlockFactor<R, true>>(L, s) : issue_op<GBlockFactor<R, false>>(L, s);
-            case G_BLOCK_SWEEP:
-                return v ? issue_op<GBlockSweep<R, true>>(L, s) : issue_op<GBlockSweep<R, false>>(L, s);
             default: fail(GLIDE_ERR_STATE, "unknown grouped launch kind");
         }
         return 0;
@@ -2231,6 +2278,7 @@ int glide_adjoint_sweep(glide_handle h, int level, double dt, int n, void* strea
         dispatch(h, [&](auto& s) {
             s.check_level(level);
             s.ensure_blocks();
+            typename std::remove_reference_t<decltype(s)>::KeepResidual keep(s);
             s.adj_sweeps(level, dt, n, S(stream));
         });
     });
@@ -2288,6 +2336,7 @@ int glide_vcycle(glide_handle h, int which, int level, int finest, double dt, vo
                 s.vcycle(level, finest != 0, dt, S(stream));
             } else {
                 s.ensure_blocks();
+                typename std::remove_reference_t<decltype(s)>::KeepResidual keep(s);
                 s.adj_vcycle(level, finest != 0, dt, S(stream));
             }
         });

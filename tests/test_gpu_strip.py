@@ -1,0 +1,95 @@
+"""The marched linear operator (glide_b200/csrc/strip.cuh) where its strips and
+chunks can go wrong: widths around the 27 and 28 owned columns and the 32 lanes,
+heights around a chunk, the smallest levels, linear and nonlinear sliding,
+calving on.
+
+J^T lambda and the fused adjoint sweeps against the oracle (binary64 1e-12 for
+one product, 1e-10 for sweeps); J e against the oracle's residual by Richardson
+-extrapolated central differences: with steps h and h/2 of the relative size
+1e-4 their truncation is O(h^4) and their rounding eps / h = 1e-12 of the
+residual's terms, which the thin columns amplify; 1e-6 as for the solver tests.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from cases import random_state
+from util import oracle_single_level, rel_err
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+DX, DT = 1500.0, 5.0
+SIZES = [(2, 2), (3, 26), (4, 27), (5, 28), (9, 31), (17, 33), (34, 55), (66, 57)]
+PHYS = [dict(calving_rate=2.0), dict(m=1.0 / 3.0)]
+
+
+def _setup(ny, nx, phys, seed=0):
+    from glide_b200.hierarchy import Hierarchy
+    f = random_state(ny, nx, seed=7 * ny + nx + seed)
+    rng = np.random.default_rng(ny + nx)
+    lam = [rng.standard_normal(s) for s in ((ny, nx + 1), (ny + 1, nx), (ny, nx))]
+    h = Hierarchy(ny, nx, DX, 1)
+    for k in ("u", "v", "H", "H_prev", "mask", "bed", "B", "beta", "smb", "f_u", "f_v"):
+        h.set(k, 0, torch.as_tensor(f[k]))
+    o = oracle_single_level({f"in_{k}": a for k, a in f.items()}, DX)
+    h.set_phys(-1, **phys)
+    o.set_phys(**phys)
+    h.compute_phi(0)
+    o.levels[0].compute_phi()
+    return h, o.levels[0], lam
+
+
+@pytest.mark.parametrize("phys", PHYS)
+@pytest.mark.parametrize("ny,nx", SIZES)
+def test_transposed_product_and_sweeps_match_oracle(ny, nx, phys):
+    h, lev, lam = _setup(ny, nx, phys)
+    rng = np.random.default_rng(5)
+    for q, k in enumerate("uvH"):
+        rhs = rng.standard_normal(lam[q].shape)
+        h.set("lambda_" + k, 0, torch.as_tensor(lam[q]))
+        h.set("adj_f_" + k, 0, torch.as_tensor(rhs))
+        getattr(lev, "l_" + k)[...] = lam[q]
+        getattr(lev, "af_" + k)[...] = rhs
+    h.vjp(0, DT)
+    for a in (lev.vjp_u, lev.vjp_v, lev.vjp_H):
+        a.fill(0)
+    lev.adj_vjp(DT)
+    for k in "uvH":
+        assert rel_err(h.view("vjp_" + k, 0).cpu().numpy(), getattr(lev, "vjp_" + k)) <= 1e-12, k
+    for n in (3, 2):  # an odd count starts in the second buffer
+        h.adjoint_sweep(0, DT, n)
+        lev.adj_sweep(DT, n)
+        for k in "uvH":
+            assert rel_err(h.view("lambda_" + k, 0).cpu().numpy(), getattr(lev, "l_" + k)) <= 1e-10, (n, k)
+            # the residual the last sweep started from stays readable
+            assert rel_err(h.view("adj_r_" + k, 0).cpu().numpy(), getattr(lev, "ar_" + k)) <= 1e-10, (n, k)
+
+
+@pytest.mark.parametrize("phys", PHYS)
+@pytest.mark.parametrize("ny,nx", SIZES)
+def test_jacobian_product_matches_differences(ny, nx, phys):
+    h, lev, e = _setup(ny, nx, phys, seed=1)
+    e[0][:, [0, -1]] = 0.0
+    e[1][[0, -1]] = 0.0
+    for q, k in enumerate("uvH"):
+        h.set("var_" + k, 0, torch.as_tensor(e[q]))
+    h.jvp(0, DT, reference_rows=True, flags=0)
+    base = [lev.u.copy(), lev.v.copy(), lev.H.copy()]
+    phi = lev.phi.copy()
+
+    def rows(s):
+        lev.u[...], lev.v[...], lev.H[...] = (b + s * d for b, d in zip(base, e))
+        lev.phi[...] = phi
+        return [a.copy() for a in lev.residual(DT, use_mask=False, operator_only=True, freeze_phi=True)]
+
+    def diff(s):
+        return [(a - b) / (2 * s) for a, b in zip(rows(s), rows(-s))]
+
+    s = 2e-3
+    want = [(4 * b - a) / 3 for a, b in zip(diff(s), diff(s / 2))]
+    want[0][:, [0, -1]] = 0.0  # pinned rows are zero in the reference's convention
+    want[1][[0, -1]] = 0.0
+    for k, w in zip("uvH", want):
+        assert rel_err(h.view("jvp_" + k, 0).cpu().numpy(), w) <= 1e-6, k
