@@ -179,8 +179,8 @@ struct SweepArgs {
     int gmode;                   // GammaMode
 };
 
-// LIN: the local iteration of local_cell.cuh (linear sliding); otherwise the
-// general local system.  A block of BY x BX threads solves one cell each: its
+// LIN: the local iteration of local_cell.cuh (linear sliding, binary32);
+// otherwise the general local system.  A block of BY x BX threads solves one cell each: its
 // own (BY - 1) x (BX - 1) cells and, redundantly, the row above and the column
 // left of them, so that it owns its faces outright.
 template <class R, bool PHI_LIVE, bool LIN, int BY, int BX, class BLK>
@@ -219,7 +219,7 @@ __device__ __forceinline__ void vanka_sweep_tile(const SweepArgs<R>& a, int gmod
         masked = own ? a.mask.at(i, j) : R(0);  // halo cells never write it
         int k = 0;
         if constexpr (LIN) {
-            LocalCell<R> cell;
+            LocalCell cell;
             cell.load(s, a.p, i, j, ldg(&a.f_u.at(i, j)), ldg(&a.f_u.at(i, j + 1)), ldg(&a.f_v.at(i, j)),
                       ldg(&a.f_v.at(i + 1, j)), ldg(&a.f_H.at(i, j)));
             R d[5] = {0, 0, 0, 0, 0};

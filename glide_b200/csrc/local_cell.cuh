@@ -16,40 +16,18 @@
 // -(ssa_damping + water_drag), which is why the caller takes this path only
 // where that sum is positive; the determinant is at least 1.
 //
-// The sweep is bound by binary64 (binary32) arithmetic and its latency, not
-// by memory: about 340 operations an iteration here against about 900 in the
-// general form (local_system + lu5_solve), which stays for m != 1.  Measured
-// per 3-V-cycle step of the reference algorithm: 64^2 31.1 -> 9.4 ms, 512^2
-// 56.5 -> 26.6 ms; binary32 600 x 424, 2 V-cycles, 19.2 -> 9.0 ms.
+// The sweep is bound by arithmetic and its latency, not by memory: about 340
+// operations an iteration here against about 900 in the general form
+// (local_system + lu5_solve).  Measured in binary32, 600 x 424, 2 V-cycles:
+// 19.2 -> 9.0 ms.  Binary32 only: see Solver::launch_sweep.
 #pragma once
 
 #include "stencil.cuh"
 
 namespace glide {
 
-// 1 / x and 1 / sqrt(x) of binary64 values of ordinary magnitude (the local
-// iteration's are: q = w^2 + 10, |D| >= damping + drag, determinant >= 1): the
-// hardware's approximation (about 20 bits) and one third-order Householder
-// step of y -> 1/y - x and of y -> 1/y^2 - x, whose error is the cube of the
-// start's, below 2^-56.  No branch for special operands, so several of them
-// overlap.  Binary32 uses the approximate instructions of its build.
-__device__ __forceinline__ double fast_rcp(double x) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-}
-__device__ __forceinline__ float fast_rcp(float x) { return 1.0f / x; }
-__device__ __forceinline__ double fast_rsqrt(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x * y, y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
-}
-__device__ __forceinline__ float fast_rsqrt(float x) { return rsqrtf(x); }
-
-template <class R>
 struct LocalCell {
+    using R = float;
     R x[5];        // unknowns at the start of the sweep
     R r0[4];       // momentum residuals of the frozen part at the start
     R dd[4];       // minus the neighbours' normal stress and drag on each row's own face
@@ -129,7 +107,7 @@ struct LocalCell {
     // q = hd (sw (H + Hn) + a (H - Hn)), a = sqrt(w^2 + 10).
     static __device__ __forceinline__ void face(R sw, R h, R Hn, R hd, R& r, R& jw, R& jh) {
         const R q2 = sw * sw + R(10);
-        const R ra = fast_rsqrt(q2);
+        const R ra = rsqrtf(q2);
         const R a = q2 * ra;
         const R sum = h + Hn, dif = h - Hn;
         r += hd * (sw * sum + a * dif);
@@ -212,11 +190,11 @@ struct LocalCell {
             // D y + (alpha, -alpha, -beta, beta) + c eta = r for the velocities,
             // alpha = G (2 s + t), beta = G (s + 2 t), s = y1 - y0, t = y2 - y3;
             // a . y + a4 eta = r4.  Pinned unknowns leave the other rows.
-            const R i0 = pin[0] ? R(0) : fast_rcp(D[0]), i1 = pin[1] ? R(0) : fast_rcp(D[1]);
-            const R i2 = pin[2] ? R(0) : fast_rcp(D[2]), i3 = pin[3] ? R(0) : fast_rcp(D[3]);
+            const R i0 = pin[0] ? R(0) : R(1) / D[0], i1 = pin[1] ? R(0) : R(1) / D[1];
+            const R i2 = pin[2] ? R(0) : R(1) / D[2], i3 = pin[3] ? R(0) : R(1) / D[3];
             const R gp = G * (i0 + i1), gq = G * (i2 + i3);
             const R m11 = R(1) - R(2) * gp, m22 = R(1) - R(2) * gq;
-            const R idet = fast_rcp(m11 * m22 - gp * gq);
+            const R idet = R(1) / (m11 * m22 - gp * gq);
             R y[4], z[4];  // y = y_r - eta z
             {
                 y[0] = i0 * r[0]; y[1] = i1 * r[1]; y[2] = i2 * r[2]; y[3] = i3 * r[3];
@@ -234,7 +212,7 @@ struct LocalCell {
             }
             const R num = r[4] - (a0 * y[0] + a1 * y[1] + a2 * y[2] + a3 * y[3]);
             const R den = a4 - (a0 * z[0] + a1 * z[1] + a2 * z[2] + a3 * z[3]);
-            const R eta = act ? R(0) : num * fast_rcp(den);
+            const R eta = act ? R(0) : num / den;
 #pragma unroll
             for (int q = 0; q < 4; ++q) d[q] -= relax * (pin[q] ? r[q] : y[q] - eta * z[q]);
             d[4] = fmax(d[4] - relax * (act ? r[4] : eta), thk - x[4]);
