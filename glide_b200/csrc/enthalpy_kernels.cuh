@@ -118,12 +118,13 @@ __device__ __forceinline__ Drain drainage(double Ek, double Ep, double drain, do
     return drain_terms(sp, s, drain, h);
 }
 
-// Lax-Friedrichs enthalpy flux through a face with mass flux q; sq = sqrt(1 + lf_c)
-// (enthalpy.cu:573-592)
-struct Flux { double res, dl, dr; };
-__device__ __forceinline__ Flux face_flux(double q, double El, double Er, double sq) {
-    double alpha = fabs(q) * sq;
-    return {0.5 * q * (El + Er) - 0.5 * alpha * (Er - El), 0.5 * (q + alpha), 0.5 * (q - alpha)};
+// Lax-Friedrichs enthalpy flux through a face with mass flux q, as the
+// coefficients of the enthalpies on its two sides: dl El + dr Er with
+// alpha = |q| sqrt(1 + lf_c) (enthalpy.cu:573-592)
+struct Flux { double dl, dr; };
+__device__ __forceinline__ Flux face_flux(double q, double sq) {
+    const double alpha = __dmul_rn(fabs(q), sq);
+    return {0.5 * (q + alpha), 0.5 * (q - alpha)};
 }
 
 // Per-column horizontal context: thicknesses of the column and its four
@@ -159,26 +160,28 @@ __device__ __forceinline__ FaceQ face_q(const EnthArgs& a, const ColumnCtx& x, i
     const double* uk = a.u + k * a.u_layer + size_t(x.i) * a.ld_u;
     const double* vk = a.v + k * a.v_layer;
     FaceQ q{0.0, 0.0, 0.0, 0.0};
+    // layer velocities come in m/s: nothing to divide, and four binary64
+    // divisions a row are a third of this function
+    const bool div = a.vel_div != 1.0;
+    auto vel = [&](double w) { return div ? w / a.vel_div : w; };
     if (x.j > 0) {
-        double ul = uk[x.j] / a.vel_div;
-        q.l = 0.5 * (x.Hxm + x.h) * ul - 0.5 * sqrt(ul * ul + kReg) * (x.h - x.Hxm);
+        double ul = vel(uk[x.j]);
+        q.l = fma(0.5 * (x.Hxm + x.h), ul, -(0.5 * sqrt(fma(ul, ul, kReg)) * (x.h - x.Hxm)));
     }
     if (x.j < a.nx - 1) {
-        double ur = uk[x.j + 1] / a.vel_div;
-        q.r = 0.5 * (x.h + x.Hxp) * ur - 0.5 * sqrt(ur * ur + kReg) * (x.Hxp - x.h);
+        double ur = vel(uk[x.j + 1]);
+        q.r = fma(0.5 * (x.h + x.Hxp), ur, -(0.5 * sqrt(fma(ur, ur, kReg)) * (x.Hxp - x.h)));
     }
     if (x.i > 0) {
-        double vt = vk[size_t(x.i) * a.ld_v + x.j] / a.vel_div;
-        q.t = 0.5 * (x.Hym + x.h) * vt - 0.5 * sqrt(vt * vt + kReg) * (x.Hym - x.h);
+        double vt = vel(vk[size_t(x.i) * a.ld_v + x.j]);
+        q.t = fma(0.5 * (x.Hym + x.h), vt, -(0.5 * sqrt(fma(vt, vt, kReg)) * (x.Hym - x.h)));
     }
     if (x.i < a.ny - 1) {
-        double vb = vk[size_t(x.i + 1) * a.ld_v + x.j] / a.vel_div;
-        q.b = 0.5 * (x.h + x.Hyp) * vb - 0.5 * sqrt(vb * vb + kReg) * (x.h - x.Hyp);
+        double vb = vel(vk[size_t(x.i + 1) * a.ld_v + x.j]);
+        q.b = fma(0.5 * (x.h + x.Hyp), vb, -(0.5 * sqrt(fma(vb, vb, kReg)) * (x.h - x.Hyp)));
     }
     return q;
 }
-
-struct HAdv { double res, diag; };
 
 // The four horizontal neighbours of node (k, i, j) in the state array; a
 // neighbour across the domain edge reads as 0 and is not used.
@@ -193,38 +196,43 @@ __device__ __forceinline__ Nbr neighbours(const EnthArgs& a, const ColumnCtx& x,
     return n;
 }
 
-// Conservative horizontal advection at (i, j, k) with centre value Ec and
-// the neighbours n read from the state array (enthalpy.cu:667-759).  sq =
-// sqrt(1 + lf_c), dx_inv = 1 / dx.
-__device__ __forceinline__ HAdv horiz_vals(const EnthArgs& a, const ColumnCtx& x, double Ec, const Nbr& n,
-                                           const FaceQ& q, double sq, double dx_inv) {
-    Flux fl = x.j > 0 ? face_flux(q.l, n.l, Ec, sq) : face_flux(0.0, Ec, Ec, sq);
-    Flux fr = x.j < a.nx - 1 ? face_flux(q.r, Ec, n.r, sq) : face_flux(0.0, Ec, Ec, sq);
-    Flux ft = x.i > 0 ? face_flux(q.t, Ec, n.t, sq) : face_flux(0.0, Ec, Ec, sq);
-    Flux fb = x.i < a.ny - 1 ? face_flux(q.b, n.b, Ec, sq) : face_flux(0.0, Ec, Ec, sq);
-    return {kRhoI * ((fr.res - fl.res) + (ft.res - fb.res)) * dx_inv,
-            kRhoI * ((fr.dl - fl.dr) + (ft.dl - fb.dr)) * dx_inv};
+// Conservative horizontal advection at (i, j, k) is linear in the centre value
+// and the four neighbours (enthalpy.cu:667-759): c Ec + l El + r Er + t Et +
+// b Eb, scaled by rho / dx.  A face on the domain edge carries no mass flux, so
+// its coefficients are zero.  c is also the term's diagonal.  Two operations a
+// neighbour and row instead of the seven of two flux evaluations.
+struct HCoef { double c, l, r, t, b; };
+__device__ __forceinline__ HCoef horiz_coef(const FaceQ& q, double sq, double scale) {
+    const Flux fl = face_flux(q.l, sq), fr = face_flux(q.r, sq), ft = face_flux(q.t, sq), fb = face_flux(q.b, sq);
+    return {scale * ((fr.dl - fl.dr) + (ft.dl - fb.dr)), -(scale * fl.dl), scale * fr.dr, scale * ft.dr,
+            -(scale * fb.dl)};
+}
+__device__ __forceinline__ double horiz_nbrs(const HCoef& h, const Nbr& n) {
+    return fma(h.r, n.r, h.l * n.l) + fma(h.t, n.t, h.b * n.b);
 }
 
-// Per-column horizontal-advection context: the hoisted face fluxes (valid
-// for every k when the velocity is layer-independent) and the constants.
+// Per-column horizontal-advection context: the coefficients, valid for every
+// k when the velocity is layer-independent, and the constants.
 struct HCtx {
-    FaceQ q;
+    HCoef h;
     bool flat;  // velocity independent of the layer
-    double sq, dx_inv;
+    double sq, scale;
     __device__ HCtx(const EnthArgs& a, const ColumnCtx& x) {
         flat = a.u_layer == 0 && a.v_layer == 0;
         sq = sqrt(1.0 + a.lf_c);
-        dx_inv = 1.0 / a.dx;
-        q = flat ? face_q(a, x, 0) : FaceQ{0.0, 0.0, 0.0, 0.0};
+        scale = kRhoI * (1.0 / a.dx);
+        h = flat ? horiz_coef(face_q(a, x, 0), sq, scale) : HCoef{0.0, 0.0, 0.0, 0.0, 0.0};
+    }
+    __device__ HCoef row(const EnthArgs& a, const ColumnCtx& x, int k) const {
+        return flat ? h : horiz_coef(face_q(a, x, k), sq, scale);
     }
 };
 
 // Vertical terms of row k < nz - 1: sigma advection, diffusion, drainage with
-// their tridiagonal coefficients (enthalpy.cu:217-509).  K_lo / K_up are the
-// diffusivities of the interfaces below and above node k, which the caller
-// carries from row to row (the reference evaluates each twice, from the same
-// arguments).
+// their tridiagonal coefficients (enthalpy.cu:217-509).  K_up is the
+// diffusivity of the interface above node k; the interface below was the row
+// before's, whose fluxes are carried (the reference evaluates each interface
+// twice, from the same arguments).
 struct Vert { double adv, dif, drn; double a, b_dif, b_adv, b_drn, c; };
 
 // Per-column constants of the vertical terms: 1 / dsig, 1 / dsig^2 and the
@@ -237,43 +245,52 @@ struct ColTerms {
         : di(1.0 / dsig), d2(1.0 / (dsig * dsig)), cold(drain_terms(c.sp_lo, c.s_lo, a.drain, h)) {}
 };
 
-__device__ __forceinline__ Vert vertical(const EnthArgs& a, int k, double Ekm1, double Ek, double Ekp1,
-                                         double Epk, double K_lo, double K_up, double om_m, double om_k,
-                                         double om_p, double h, double h_inv, double dsig, const Clamped& cl,
-                                         const ColTerms& ct) {
+// What the interface above a row hands to the row above it: the advective flux
+// and its two one-sided speeds, the diffusive flux and its coefficient.
+struct Iface { double F, p, n, D, dk; };
+
+__device__ __forceinline__ Vert vertical(const EnthArgs& a, int k, double Ek, double Ekp1, double Epk, double K_up,
+                                         double om_k, double om_p, double h, double h_inv, double dsig,
+                                         const Clamped& cl, const ColTerms& ct, Iface& lo) {
     Vert r{0, 0, 0, 0, 0, 0, 0, 0};
+    Iface up{0, 0, 0, 0, 0};
+    if (a.flags & kTermSigmaDot) {
+        const double w = 0.5 * (om_k + om_p);
+        up.p = fmax(w, 0.0);
+        up.n = fmin(w, 0.0);
+        up.F = fma(up.p, Ek, up.n * Ekp1);
+    }
+    // products that are also carried are rounded here, so that every compiled
+    // form of the smoother sums the same numbers
+    up.D = __dmul_rn(K_up, Ekp1 - Ek);
     if (k == 0) {
         const double dsh = 0.5 * dsig, dsh_inv = 1.0 / dsh;
         if (a.flags & kTermSigmaDot) {
-            double wh = 0.5 * (om_k + om_p);
-            double wp = fmax(wh, 0.0), wn = fmin(wh, 0.0);
-            double Fu = wp * Ek + wn * Ekp1, Fb = om_k * Ek;
-            r.adv = kRhoI * (Fu - Fb) * dsh_inv;
-            r.b_adv = kRhoI * (wp - om_k) * dsh_inv;
-            r.c = kRhoI * wn * dsh_inv;
+            r.adv = kRhoI * (up.F - om_k * Ek) * dsh_inv;
+            r.b_adv = kRhoI * (up.p - om_k) * dsh_inv;
+            r.c = kRhoI * up.n * dsh_inv;
         }
-        r.dif = (-h_inv * K_up * (Ekp1 - Ek) / dsig - 0.0) / dsh;
-        double coeff = h_inv * K_up / (dsig * dsh);
+        r.dif = (-h_inv * up.D / dsig - 0.0) / dsh;
+        const double coeff = h_inv * K_up / (dsig * dsh);
         r.b_dif = coeff;
         r.c += -coeff;
+        up.dk = __dmul_rn(h_inv * ct.d2, K_up);
     } else {
-        const double di = ct.di;
+        const double s = kRhoI * ct.di;
         if (a.flags & kTermSigmaDot) {
-            double wu = 0.5 * (om_k + om_p), wl = 0.5 * (om_m + om_k);
-            double up = fmax(wu, 0.0), un = fmin(wu, 0.0), lp = fmax(wl, 0.0), ln = fmin(wl, 0.0);
-            double Fu = up * Ek + un * Ekp1, Fl = lp * Ekm1 + ln * Ek;
-            r.adv = kRhoI * (Fu - Fl) * di;
-            r.a = -kRhoI * lp * di;
-            r.c = kRhoI * un * di;
-            r.b_adv = kRhoI * (up - ln) * di;
+            r.adv = s * (up.F - lo.F);
+            r.a = -s * lo.p;
+            r.c = s * up.n;
+            r.b_adv = s * (up.p - lo.n);
         }
-        const double d2 = ct.d2;
-        r.dif = -h_inv * d2 * (K_up * (Ekp1 - Ek) - K_lo * (Ek - Ekm1));
-        double dl = h_inv * d2 * K_lo, du = h_inv * d2 * K_up;
-        r.a += -dl;
-        r.c += -du;
-        r.b_dif = dl + du;
+        const double hd = h_inv * ct.d2;
+        r.dif = -hd * (up.D - lo.D);
+        up.dk = __dmul_rn(hd, K_up);
+        r.a += -lo.dk;
+        r.c += -up.dk;
+        r.b_dif = lo.dk + up.dk;
     }
+    lo = up;
     if (a.flags & kTermDrainage) {
         Drain d = drainage(Ek, Epk, a.drain, h, cl, ct.cold);
         r.drn = d.res;
@@ -304,12 +321,6 @@ __device__ __forceinline__ RowIn row_inputs(const EnthArgs& a, const ColumnCtx& 
 }
 __device__ __forceinline__ RowIn no_row() { return RowIn{0.0, 0.0, 0.0, Nbr{0.0, 0.0, 0.0, 0.0}}; }
 
-// Horizontal advection of row k from its loaded neighbours.
-__device__ __forceinline__ HAdv row_horiz(const EnthArgs& a, const ColumnCtx& x, const HCtx& hc, int k, double Ec,
-                                          const Nbr& nb) {
-    return horiz_vals(a, x, Ec, nb, hc.flat ? hc.q : face_q(a, x, k), hc.sq, hc.dx_inv);
-}
-
 // ------------------------------------------------------------- residual
 // enthalpy.cu:784-893.  out (layer-major) = F(E) - f_E, or F(E) without
 // forcing; partial[block] = max |out| over the block's nodes.
@@ -334,10 +345,10 @@ __global__ void __launch_bounds__(kColThreads, MINB) k_enth_residual(EnthArgs a,
             const ColTerms ct(a, cl, x.h, dsig);
             const double* E = a.E + x.c;
             const double* om = a.omega + x.c;
-            double Ekm1 = 0.0, Ek = E[0], Ekp1 = E[plane];
+            double Ek = E[0], Ekp1 = E[plane];
             double Epk = e_pmp(0.0, x.h), Epp = e_pmp(dsig, x.h);
-            double K_lo = 0.0;
-            double om_m = 0.0, om_k = om[0];
+            Iface lo{0, 0, 0, 0, 0};
+            double om_k = om[0];
             const bool hadv = (a.flags & kTermHorizAdv) != 0;
             RowIn in = row_inputs(a, x, 0, hadv, use_forcing);
             for (int k = 0; k < nz - 1; ++k) {
@@ -346,8 +357,11 @@ __global__ void __launch_bounds__(kColThreads, MINB) k_enth_residual(EnthArgs a,
                 const double om_p = in.om_p;
                 const double K_up = k_diff(0.5 * (Ek + Ekp1), 0.5 * (Epk + Epp), cl);
                 double r = kRhoI * (x.h * Ek - x.h_prev * in.ep) * inv_dt;
-                if (hadv) r += row_horiz(a, x, hc, k, Ek, in.nb).res;
-                Vert vt = vertical(a, k, Ekm1, Ek, Ekp1, Epk, K_lo, K_up, om_m, om_k, om_p, x.h, x.h_inv, dsig, cl, ct);
+                if (hadv) {
+                    const HCoef hk = hc.row(a, x, k);
+                    r += hk.c * Ek + horiz_nbrs(hk, in.nb);
+                }
+                Vert vt = vertical(a, k, Ek, Ekp1, Epk, K_up, om_k, om_p, x.h, x.h_inv, dsig, cl, ct, lo);
                 r += vt.adv;
                 r += vt.dif;
                 r += vt.drn;
@@ -355,11 +369,10 @@ __global__ void __launch_bounds__(kColThreads, MINB) k_enth_residual(EnthArgs a,
                 out[k * plane + x.c] = r;
                 mx = fmax(mx, fabs(r));
                 // slide the window
-                Ekm1 = Ek; Ek = Ekp1; Ekp1 = E_n;
+                Ek = Ekp1; Ekp1 = E_n;
                 Epk = Epp;
                 Epp = e_pmp(double(k + 2 < nz ? k + 2 : nz - 1) * dsig, x.h);
-                K_lo = K_up;
-                om_m = om_k; om_k = om_p;
+                om_k = om_p;
                 in = in_n;
             }
             out[size_t(nz - 1) * plane + x.c] = 0.0;
@@ -415,11 +428,12 @@ __global__ void __launch_bounds__(kColThreads, MINB) k_enth_column(EnthArgs a, d
     const bool hadv = (a.flags & kTermHorizAdv) != 0;
     for (int it = 0; it < a.n_newton; ++it) {
         double Epk = e_pmp(0.0, x.h), Epp = e_pmp(dsig, x.h);
-        double K_lo = 0.0, om_m = 0.0, om_k = om[0];
+        double om_k = om[0];
+        Iface lo{0, 0, 0, 0, 0};
         double c_prev = 0.0, d_prev = 0.0;
         // the iterate window of row k and the inputs of row k + 1 are
         // loaded before row k is assembled
-        double Ekm1 = 0.0, Ek = El[0], Ekp1 = El[1];
+        double Ek = El[0], Ekp1 = El[1];
         RowIn in = row_inputs(a, x, 0, hadv, true);
         for (int k = 0; k < nz - 1; ++k) {
             const RowIn in_n = k + 1 < nz - 1 ? row_inputs(a, x, k + 1, hadv, true) : no_row();
@@ -429,11 +443,11 @@ __global__ void __launch_bounds__(kColThreads, MINB) k_enth_column(EnthArgs a, d
             double r = kRhoI * (x.h * Ek - x.h_prev * in.ep) * inv_dt - in.fe;
             double hd = 0.0;
             if (hadv) {
-                HAdv ha = row_horiz(a, x, hc, k, Ek, in.nb);
-                r += ha.res;
-                hd = ha.diag;
+                const HCoef hk = hc.row(a, x, k);
+                r += hk.c * Ek + horiz_nbrs(hk, in.nb);
+                hd = hk.c;
             }
-            Vert vt = vertical(a, k, Ekm1, Ek, Ekp1, Epk, K_lo, K_up, om_m, om_k, om_p, x.h, x.h_inv, dsig, cl, ct);
+            Vert vt = vertical(a, k, Ek, Ekp1, Epk, K_up, om_k, om_p, x.h, x.h_inv, dsig, cl, ct, lo);
             r += vt.adv;
             r += vt.dif;
             r += vt.drn;
@@ -447,9 +461,8 @@ __global__ void __launch_bounds__(kColThreads, MINB) k_enth_column(EnthArgs a, d
             dp[k] = d_prev;
             Epk = Epp;
             Epp = e_pmp(double(k + 2 < nz ? k + 2 : nz - 1) * dsig, x.h);
-            K_lo = K_up;
-            om_m = om_k; om_k = om_p;
-            Ekm1 = Ek; Ek = Ekp1; Ekp1 = E_n;
+            om_k = om_p;
+            Ek = Ekp1; Ekp1 = E_n;
             in = in_n;
         }
         // surface Dirichlet row: E = E_surface (a = c = 0, b = 1)
@@ -512,9 +525,10 @@ __device__ __forceinline__ void column_newton_step(const EnthArgs& a, const Colu
     const double* om = a.omega + x.c;
     const double* src = FIRST ? E : El;
     double Epk = e_pmp(0.0, x.h), Epp = e_pmp(dsig, x.h);
-    double K_lo = 0.0, om_m = 0.0, om_k = om[0];
+    double om_k = om[0];
+        Iface lo{0, 0, 0, 0, 0};
     double c_prev = 0.0, d_prev = 0.0;
-    double Ekm1 = 0.0, Ek = src[0], Ekp1 = src[plane];
+    double Ek = src[0], Ekp1 = src[plane];
     // row k + 1's inputs are loaded while row k is assembled
     RowIn in = FIRST ? row_inputs(a, x, 0, cs.hadv, true) : no_row();
     double Cn = FIRST ? 0.0 : C[0];
@@ -527,7 +541,7 @@ __device__ __forceinline__ void column_newton_step(const EnthArgs& a, const Colu
             if (k + 1 < nz - 1) in_n = row_inputs(a, x, k + 1, cs.hadv, true);
             // the row constant: old time level, forcing, frozen neighbours
             ck = -cs.ct_old * in.ep - in.fe;
-            if (cs.fold) ck += row_horiz(a, x, hc, k, 0.0, in.nb).res;
+            if (cs.fold) ck += horiz_nbrs(hc.h, in.nb);
             C[size_t(k) * plane] = ck;
             om_p = in.om_p;
         } else {
@@ -545,11 +559,11 @@ __device__ __forceinline__ void column_newton_step(const EnthArgs& a, const Colu
             r += cs.hd_flat * Ek;
         } else if (cs.hadv) {
             const Nbr nb = FIRST ? in.nb : neighbours(a, x, k);
-            HAdv ha = row_horiz(a, x, hc, k, Ek, nb);
-            r += ha.res;
-            hd = ha.diag;
+            const HCoef hk = hc.row(a, x, k);
+            r += hk.c * Ek + horiz_nbrs(hk, nb);
+            hd = hk.c;
         }
-        Vert vt = vertical(a, k, Ekm1, Ek, Ekp1, Epk, K_lo, K_up, om_m, om_k, om_p, x.h, x.h_inv, dsig, cl, ct);
+        Vert vt = vertical(a, k, Ek, Ekp1, Epk, K_up, om_k, om_p, x.h, x.h_inv, dsig, cl, ct, lo);
         r += vt.adv;
         r += vt.dif;
         r += vt.drn;
@@ -563,9 +577,8 @@ __device__ __forceinline__ void column_newton_step(const EnthArgs& a, const Colu
         Dp[size_t(k) * plane] = d_prev;
         Epk = Epp;
         Epp = e_pmp(double(k + 2 < nz ? k + 2 : nz - 1) * dsig, x.h);
-        K_lo = K_up;
-        om_m = om_k; om_k = om_p;
-        Ekm1 = Ek; Ek = Ekp1; Ekp1 = E_n;
+        om_k = om_p;
+        Ek = Ekp1; Ekp1 = E_n;
         if (FIRST) in = in_n;
     }
     // surface Dirichlet row: E = E_surface (a = c = 0, b = 1), then back
@@ -591,34 +604,34 @@ __device__ __forceinline__ void column_newton_step(const EnthArgs& a, const Colu
         pd[q] = k >= 0 ? Dp[size_t(k) * plane] : 0.0;
         pe[q] = (want_e && k >= 0) ? E[size_t(k) * plane] : 0.0;
     }
-#pragma unroll kPre
-    for (int q = 0; q < nz - 1; ++q) {
-        const int k = nz - 2 - q, slot = q % kPre;
-        const double sk = ps[slot], dk = pd[slot], ek = pe[slot];
-        const int kn = k - kPre;
-        if (kn >= 0) {
-            ps[slot] = src[size_t(kn) * plane];
-            pd[slot] = Dp[size_t(kn) * plane];
-            if (want_e) pe[slot] = E[size_t(kn) * plane];
-        }
-        xk = dk - cps[size_t(k) * bd] * xk;
-        en = sk + a.relaxation * xk;
-        if (last) {
-            const double E0 = FIRST ? sk : ek;
-            El[size_t(k) * plane] = mode ? E0 + a.omega_relax * (en - E0) : en - E0;
-        } else {
-            El[size_t(k) * plane] = en;
+    // groups of kPre rows, so that every ring slot is a register
+    for (int q0 = 0; q0 < nz - 1; q0 += kPre) {
+#pragma unroll
+        for (int slot = 0; slot < kPre; ++slot) {
+            const int k = nz - 2 - (q0 + slot);
+            if (k < 0) break;
+            const double sk = ps[slot], dk = pd[slot], ek = pe[slot];
+            const int kn = k - kPre;
+            if (kn >= 0) {
+                ps[slot] = src[size_t(kn) * plane];
+                pd[slot] = Dp[size_t(kn) * plane];
+                if (want_e) pe[slot] = E[size_t(kn) * plane];
+            }
+            xk = dk - cps[size_t(k) * bd] * xk;
+            en = sk + a.relaxation * xk;
+            if (last) {
+                const double E0 = FIRST ? sk : ek;
+                El[size_t(k) * plane] = mode ? E0 + a.omega_relax * (en - E0) : en - E0;
+            } else {
+                El[size_t(k) * plane] = en;
+            }
         }
     }
 }
 
-template <int MINB>
-__global__ void __launch_bounds__(kColSmemThreads, MINB)
-    k_enth_column_s(EnthArgs a, double* out, double* rowc, double* dpr, int mode) {
-    extern __shared__ double sm[];
-    if (stopped(a.done)) return;
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= a.ny * a.nx) return;
+// One column of the smoother.
+__device__ __forceinline__ void column_s(const EnthArgs& a, int col, double* out, double* rowc, double* dpr,
+                                         double* sm, int mode) {
     const int nz = a.nz;
     const size_t plane = size_t(a.ny) * a.nx;
     const int i = col / a.nx, j = col % a.nx;
@@ -650,7 +663,7 @@ __global__ void __launch_bounds__(kColSmemThreads, MINB)
     cs.ct_old = kRhoI * x.h_prev * inv_dt;  // time-term weight of E_prev
     cs.hadv = (a.flags & kTermHorizAdv) != 0;
     cs.fold = cs.hadv && hc.flat;           // horizontal flux folded into the row constants
-    cs.hd_flat = cs.fold ? horiz_vals(a, x, 0.0, Nbr{0.0, 0.0, 0.0, 0.0}, hc.q, hc.sq, hc.dx_inv).diag : 0.0;
+    cs.hd_flat = cs.fold ? hc.h.c : 0.0;
     cs.Es = Es;
     double* C = rowc + x.c;
     double* Dp = dpr + x.c;
@@ -659,14 +672,19 @@ __global__ void __launch_bounds__(kColSmemThreads, MINB)
         column_newton_step<false>(a, x, cl, hc, ct, cs, E, El, C, Dp, cps, blockDim.x, it + 1 == a.n_newton, mode);
 }
 
+template <int MINB>
+__global__ void __launch_bounds__(kColSmemThreads, MINB)
+    k_enth_column_s(EnthArgs a, double* out, double* rowc, double* dpr, int mode) {
+    extern __shared__ double sm[];
+    if (stopped(a.done)) return;
+    const int col = blockIdx.x * blockDim.x + threadIdx.x;
+    if (col < a.ny * a.nx) column_s(a, col, out, rowc, dpr, sm, mode);
+}
+
 // ---------------------------------------------------------- layer smoother
 // enthalpy.cu:1129-1258: pointwise Jacobi, delta = -r / J_kk.  One thread per
 // column walking k.  mode 0 writes delta_E, mode 1 the updated state.
-template <int MINB>
-__global__ void __launch_bounds__(kColThreads, MINB) k_enth_layer(EnthArgs a, double* out, int mode) {
-    if (stopped(a.done)) return;
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= a.ny * a.nx) return;
+__device__ __forceinline__ void layer_column(const EnthArgs& a, int col, double* out, int mode) {
     const int nz = a.nz;
     const size_t plane = size_t(a.ny) * a.nx;
     const int i = col / a.nx, j = col % a.nx;
@@ -681,9 +699,10 @@ __global__ void __launch_bounds__(kColThreads, MINB) k_enth_layer(EnthArgs a, do
     const double dsig = 1.0 / double(nz - 1), inv_dt = 1.0 / a.dt;
     const ColTerms ct(a, cl, x.h, dsig);
     const double* om = a.omega + x.c;
-    double Ekm1 = 0.0, Ek = E[0], Ekp1 = E[plane];
+    double Ek = E[0], Ekp1 = E[plane];
     double Epk = e_pmp(0.0, x.h), Epp = e_pmp(dsig, x.h);
-    double K_lo = 0.0, om_m = 0.0, om_k = om[0];
+    double om_k = om[0];
+        Iface lo{0, 0, 0, 0, 0};
     const bool hadv = (a.flags & kTermHorizAdv) != 0;
     RowIn in = row_inputs(a, x, 0, hadv, true);
     for (int k = 0; k < nz - 1; ++k) {
@@ -695,26 +714,32 @@ __global__ void __launch_bounds__(kColThreads, MINB) k_enth_layer(EnthArgs a, do
         double r = kRhoI * (x.h * Ek - x.h_prev * in.ep) * inv_dt - in.fe;
         double diag = kRhoI * x.h * inv_dt;
         if (hadv) {
-            HAdv ha = row_horiz(a, x, hc, k, Ek, in.nb);
-            r += ha.res;
-            diag += ha.diag;
+            const HCoef hk = hc.row(a, x, k);
+            r += hk.c * Ek + horiz_nbrs(hk, in.nb);
+            diag += hk.c;
         }
-        Vert vt = vertical(a, k, Ekm1, Ek, Ekp1, Epk, K_lo, K_up, om_m, om_k, om_p, x.h, x.h_inv, dsig, cl, ct);
+        Vert vt = vertical(a, k, Ek, Ekp1, Epk, K_up, om_k, om_p, x.h, x.h_inv, dsig, cl, ct, lo);
         r += vt.adv;
         r += vt.dif;
         r += vt.drn;
         diag += vt.b_dif + vt.b_adv + vt.b_drn;
         const double d = (fabs(diag) > 1e-30) ? (-r / diag) : 0.0;
         out[n] = mode ? Ek + a.omega_relax * d : d;
-        Ekm1 = Ek; Ek = Ekp1; Ekp1 = E_n;
+        Ek = Ekp1; Ekp1 = E_n;
         Epk = Epp;
         Epp = e_pmp(double(k + 2 < nz ? k + 2 : nz - 1) * dsig, x.h);
-        K_lo = K_up;
-        om_m = om_k; om_k = om_p;
+        om_k = om_p;
         in = in_n;
     }
     const size_t top = size_t(nz - 1) * plane + x.c;
     out[top] = mode ? E[size_t(nz - 1) * plane] : 0.0;
+}
+
+template <int MINB>
+__global__ void __launch_bounds__(kColThreads, MINB) k_enth_layer(EnthArgs a, double* out, int mode) {
+    if (stopped(a.done)) return;
+    const int col = blockIdx.x * blockDim.x + threadIdx.x;
+    if (col < a.ny * a.nx) layer_column(a, col, out, mode);
 }
 
 // ------------------------------------------------------------ omega
@@ -835,12 +860,13 @@ __global__ void __launch_bounds__(kColThreads, 8) k_enth_arrhenius(EnthArgs a, d
         const double depth = (1.0 - sig) * h;
         const double T_pmp = 273.15 - cc * depth;
         const double Ek = a.E[size_t(k) * plane + c];
-        const double T = fmin(Ek * E_SCALE / 2009.0 + 223.15, T_pmp);
+        const double T = fmin(Ek * (E_SCALE / 2009.0) + 223.15, T_pmp);
         const bool cold = T < 263.15;
         const double Af = cold ? 3.985e-13 : 1.916e3, Qf = cold ? 60e3 : 139e3;
         double A = Af * exp(-Qf / (8.314 * fmax(T, 1.0)));
-        const double w = fmax(Ek * E_SCALE - 2009.0 * (T_pmp - 223.15), 0.0) / 334000.0;
-        return A * (1.0 + 181.25 * w);
+        // water content: none in cold ice, and no division then
+        const double x = Ek * E_SCALE - 2009.0 * (T_pmp - 223.15);
+        return x > 0.0 ? A * (1.0 + 181.25 * (x / 334000.0)) : A;
     };
     // numpy's pairwise sum of a short contiguous axis: below 8 terms in order;
     // else 8 interleaved partial sums combined pairwise, then the rest in order
