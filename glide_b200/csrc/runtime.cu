@@ -23,6 +23,7 @@
 #include "glide_b200.h"
 #include "forward_kernels.cuh"
 #include "adjoint_kernels.cuh"
+#include "adjoint_tile.cuh"
 #include "strip.cuh"
 #include "transfer_kernels.cuh"
 #include "group.cuh"
@@ -234,8 +235,9 @@ struct Solver : SolverBase {
     double* norms_host = nullptr;
     int* err_dev = nullptr;  // kStage* bits set by a staging block (its wait gave up, or its maps failed their check)
     // TMA tensor maps of every (level, field), encoded on first use
-    std::vector<CUtensorMap> tmaps;
-    std::vector<unsigned char> tmap_done;
+    // (slot 0: kBoxH rows, slot 1: the adjoint tile's)
+    std::vector<CUtensorMap> tmaps[2];
+    std::vector<unsigned char> tmap_done[2];
     bool use_tma = true;
     int tma_wait_polls = kTmaWaitPolls;  // 0 under GLIDE_TUNE_TMA_GIVE_UP
     // one captured V-cycle per cycle kind (0 FAS, 1 adjoint, 2 mixed FAS,
@@ -252,6 +254,8 @@ struct Solver : SolverBase {
     };
     CachedGraph graphs[kKinds];
     cudaStream_t own_stream = nullptr;
+    bool shadow = false;           // the binary32 half of a mixed handle
+    bool fixed_cycles = false;     // ... whose adjoint solve runs a fixed number of cycles (adjoint_tile.cuh)
     long long launches = 0;        // kernels issued by this handle (graph replays included)
     long long* launch_sink = nullptr;  // a binary32 shadow also counts into its handle's solver
     // Algorithmic bytes of those kernels: the values each must read and write
@@ -516,40 +520,41 @@ struct Solver : SolverBase {
     }
 
     // TMA staging needs a level at least one box wide and high
-    bool tma_level(int l) const { return use_tma && lv[l].nx >= kBoxW && lv[l].ny >= kBoxH; }
+    bool tma_level(int l, int bh) const { return use_tma && lv[l].nx >= kBoxW && lv[l].ny >= bh; }
 
-    const CUtensorMap& tmap(int l, int f) {
-        if (tmaps.empty()) {
-            tmaps.resize(size_t(n_levels) * F_COUNT);
-            tmap_done.assign(size_t(n_levels) * F_COUNT, 0);
+    const CUtensorMap& tmap(int l, int f, int bh) {
+        const int w = bh == kBoxH ? 0 : 1;
+        if (tmaps[w].empty()) {
+            tmaps[w].resize(size_t(n_levels) * F_COUNT);
+            tmap_done[w].assign(size_t(n_levels) * F_COUNT, 0);
         }
         const size_t k = size_t(l) * F_COUNT + f;
-        if (!tmap_done[k]) {
+        if (!tmap_done[w][k]) {
             PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
             if (!enc) fail(GLIDE_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
             const Arr<R>& a = lv[l].a[f];
             const cuuint64_t dims[2] = {cuuint64_t(a.cols), cuuint64_t(a.rows)};
             const cuuint64_t strides[1] = {cuuint64_t(a.pitch) * sizeof(R)};
-            const cuuint32_t box[2] = {cuuint32_t(kBoxW), cuuint32_t(kBoxH)};
+            const cuuint32_t box[2] = {cuuint32_t(kBoxW), cuuint32_t(bh)};
             const cuuint32_t estr[2] = {1, 1};
-            const CUresult r = enc(&tmaps[k], sizeof(R) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64
+            const CUresult r = enc(&tmaps[w][k], sizeof(R) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64
                                                                   : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
                                    2, a.p, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             if (r != CUDA_SUCCESS) fail(GLIDE_ERR_CUDA, "cuTensorMapEncodeTiled failed");
-            tmap_done[k] = 1;
+            tmap_done[w][k] = 1;
         }
-        return tmaps[k];
+        return tmaps[w][k];
     }
 
     template <int N>
-    BoxMaps<N> box_maps(int l, const int (&fields)[N]) {
+    BoxMaps<N> box_maps(int l, const int (&fields)[N], int bh = kBoxH) {
         BoxMaps<N> m;
-        m.use = tma_level(l) ? 1 : 0;
+        m.use = tma_level(l, bh) ? 1 : 0;
         m.wait_polls = tma_wait_polls;
         if (m.use)
-            for (int q = 0; q < N; ++q) m.m[q] = tmap(l, fields[q]);
+            for (int q = 0; q < N; ++q) m.m[q] = tmap(l, fields[q], bh);
         return m;
     }
 
@@ -614,12 +619,13 @@ struct Solver : SolverBase {
 
     void launch_sweep(const SweepArgs<R>& a, bool phi_live, cudaStream_t s, double bytes) {
         // The linear-sliding form reorders the local system's sums and divides
-        // by diagonals of at least damping + drag (local_cell.cuh).  Binary64
-        // keeps the general form: the local iteration stops on a threshold, a
-        // reordered sum flips a cell's count there now and then (measured in 2
-        // of 26 adjoint runs at 512^2, up to 4e-9 in the gradients), and
-        // binary64 promises the reference's iterates.
-        const bool linear = sizeof(R) == 4 && a.p.m == R(1) && a.ssa_damping + a.p.water_drag > R(0);
+        // by diagonals of at least damping + drag (local_cell.cuh).  It runs on
+        // binary32 handles only.  Binary64 and mixed handles promise the
+        // reference's binary64 iterates: there the local iteration stops on a
+        // threshold at which a reordered sum flips a cell's count now and then
+        // (2 of 26 adjoint runs at 512^2, up to 4e-9 in the gradients), and a
+        // fixed number of mixed cycles carries its shadow's rounding (6e-6).
+        const bool linear = sizeof(R) == 4 && !shadow && a.p.m == R(1) && a.ssa_damping + a.p.water_drag > R(0);
         const int form = linear ? S_LINEAR : (sweep_blocks_per_sm >= 2 ? S_GENERAL_2 : S_GENERAL_1);
         with_sweep_form<R>(form, [&](auto f) {
             launch_sweep_form<decltype(f)>(a, phi_live, (phi_live ? 1 : 0) | 2 * form, s, bytes);
@@ -808,6 +814,8 @@ struct Solver : SolverBase {
         f.quirks = quirks;
         f.sweep_blocks_per_sm = sweep_blocks_per_sm;
         f.use_graphs = 0;
+        f.shadow = true;
+        f.fixed_cycles = !(fas[1].relative_tolerance > 0.0) && !(fas[1].absolute_tolerance > 0.0);
         f.use_tma = use_tma;
         f.tma_wait_polls = tma_wait_polls;
         f.err_dev = err_dev;  // shadow kernels report into this handle's error word
@@ -1069,6 +1077,18 @@ struct Solver : SolverBase {
     void lin_op(int l, double dt, const Lin& L, const int* out, const int* sub, bool use_forcing, bool norms,
                 bool ref_rows, cudaStream_t s, int jvp_flags = GLIDE_USE_MASK) {
         StripArgs<R> q = strip_args(l, dt, L, out, sub, use_forcing, norms, ref_rows, jvp_flags);
+        if constexpr (sizeof(R) == 4) {
+            if (L.tr && fixed_cycles) {
+                const int fl[AdjTile<R>::NB] = {GLIDE_U, GLIDE_V, GLIDE_H, GLIDE_PHI, GLIDE_BED, GLIDE_BETA,
+                                                GLIDE_B, L.x[0], L.x[1]};
+                not_recordable("the tiled transposed product");
+                q.a.err = err_dev;
+                k_vjp<R><<<dim3(lv[l].blocks_x(), lv[l].blocks_y()), kTile * kTile, 0, s>>>(
+                    q.a, box_maps(l, fl, AdjTile<R>::BH));
+                counted("vjp", lb(l, 11 + (use_forcing ? 3 : 0) + (sub ? 3 : 0) + 3));
+                return;
+            }
+        }
         const dim3 g = strip_grid<false>(q);
         // u, v, H, phi, mask, bed, beta, B and the three unknowns read, the
         // forcing and the subtrahend when given, three rows written
@@ -1146,6 +1166,14 @@ struct Solver : SolverBase {
         if (factor) block_factor(l, dt, L, s);
         if (blk.empty()) fail(GLIDE_ERR_STATE, "block factor buffers not allocated");
         Level<R>& v = lv[l];
+        if (L.tr && fixed_cycles) {  // (adjoint_tile.cuh)
+            const BlockArgs<R> a = block_args(l, dt, L);
+            for (int k = 0; k < n; ++k) {
+                lin_residual(l, dt, L, false, s);
+                block_sweep(l, a, true, dim3(v.blocks_x(), v.blocks_y()), s);
+            }
+            return;
+        }
         const int alt[3] = {F_XA_U, F_XA_V, F_XA_H};
         StripArgs<R> q = strip_args(l, dt, L, nullptr, nullptr, true, false, false, GLIDE_USE_MASK);
         q.fac = blk[l];

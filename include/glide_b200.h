@@ -170,7 +170,9 @@ int glide_alg_bytes(glide_handle h, double* bytes);
  * instrumentation. */
 int glide_block_smoother_part(glide_handle h, int level, double dt, int adjoint, int part, void* stream);
 /* Kernel tuning knobs (no counterpart in the reference).
- * GLIDE_TUNE_SWEEP_BLOCKS_PER_SM: 1 or 2 resident Vanka-sweep blocks per SM.
+ * GLIDE_TUNE_SWEEP_BLOCKS_PER_SM: register budget of the general Vanka sweep:
+ * 1 = fewer resident blocks per SM with more registers each, 2 (default) =
+ * more.
  * GLIDE_TUNE_MIXED_INNER_VCYCLES: binary32 V-cycles per defect correction
  * of a GLIDE_MIXED handle (default 1). */
 #define GLIDE_TUNE_SWEEP_BLOCKS_PER_SM 1
