@@ -1,13 +1,18 @@
 // adjoint_tile.cuh -- the transposed product of one 16 x 16 tile, in the order
 // of the reference's rows.
 //
-// strip.cuh runs the transposed product everywhere but in one place: a mixed
-// handle's adjoint solve with both tolerances zero.  Such a solve returns the
-// iterate after a fixed number of cycles, whose low-order digits are the
-// binary32 shadow's rounding; summed in the march's order they differ by 2e-7
-// to 4e-6 (1 to 3 cycles, 64^2 to 560^2).  A caller that fixes the cycles gets
-// the same iterates as before, at this kernel's price (264 against 93 us at
-// 2048^2); a solve to a tolerance takes the march.
+// strip.cuh runs the linear operator everywhere but in one place: a mixed
+// handle's solves with both tolerances zero, adjoint (here, on the binary32 and
+// the binary64 half) and forward (tangent_tile.cuh, on the binary32 half, which
+// solves the tangent systems).  Such a solve returns the iterate of its last
+// cycle, whose low-order digits are the binary32 rounding of these sums.  The
+// march adds the same terms in another order, no less exact, but the iterates
+// move: a gradient by 2e-7 to 4e-6 of its norm with the binary32 half marched,
+// by up to 3e-8 with the binary64 half alone, a velocity by up to 8e-6 after two
+// forward steps (1 to 3 cycles, 64^2 to 560^2).  A caller that fixes the cycles
+// asks for that iterate, so it keeps the one it had, at this kernel's price (264
+// against 93 us for the binary32 product of 2048^2); a solve to a tolerance
+// takes the march.
 //
 // The reference forms lambda^T dR/dx by scattering every residual row's partials
 // with atomics (residuals.cu:667-1163).  Here each output entry gathers the same

@@ -25,6 +25,7 @@
 #include "adjoint_kernels.cuh"
 #include "adjoint_tile.cuh"
 #include "strip.cuh"
+#include "tangent_tile.cuh"
 #include "transfer_kernels.cuh"
 #include "group.cuh"
 
@@ -255,7 +256,10 @@ struct Solver : SolverBase {
     CachedGraph graphs[kKinds];
     cudaStream_t own_stream = nullptr;
     bool shadow = false;           // the binary32 half of a mixed handle
-    bool fixed_cycles = false;     // ... whose adjoint solve runs a fixed number of cycles (adjoint_tile.cuh)
+    // The linear operators of these systems ([1] adjoint, [2] tangent) keep the
+    // reference's row order: both halves of a mixed handle in a solve of a fixed
+    // number of cycles (adjoint_tile.cuh)
+    bool tile_order[3] = {false, false, false};
     long long launches = 0;        // kernels issued by this handle (graph replays included)
     long long* launch_sink = nullptr;  // a binary32 shadow also counts into its handle's solver
     // Algorithmic bytes of those kernels: the values each must read and write
@@ -808,6 +812,11 @@ struct Solver : SolverBase {
         counted("convert", double(src.rows) * src.cols * (sizeof(D) + sizeof(Src)));
     }
 
+    // A solve without a tolerance: it returns the iterate of its last cycle.
+    bool runs_fixed_cycles(int cfg) const {
+        return !(fas[cfg].relative_tolerance > 0.0) && !(fas[cfg].absolute_tolerance > 0.0);
+    }
+
     void sync_shadow() {
         Solver<float>& f = *lo;
         for (int q = 0; q < 3; ++q) f.fas[q] = fas[q];
@@ -815,7 +824,8 @@ struct Solver : SolverBase {
         f.sweep_blocks_per_sm = sweep_blocks_per_sm;
         f.use_graphs = 0;
         f.shadow = true;
-        f.fixed_cycles = !(fas[1].relative_tolerance > 0.0) && !(fas[1].absolute_tolerance > 0.0);
+        f.tile_order[1] = runs_fixed_cycles(1);
+        f.tile_order[2] = runs_fixed_cycles(0);  // the tangent system belongs to the forward solve
         f.use_tma = use_tma;
         f.tma_wait_polls = tma_wait_polls;
         f.err_dev = err_dev;  // shadow kernels report into this handle's error word
@@ -895,6 +905,13 @@ struct Solver : SolverBase {
 
     void backward_mixed(double dt, int start, int grad_mask, glide_stats* st, cudaStream_t s) {
         sync_shadow();
+        // the binary64 half's order is this solve's alone: the operator calls
+        // on the handle take the march whatever was solved before
+        struct TileOrder {
+            bool& on;
+            TileOrder(bool& x, bool v) : on(x) { on = v; }
+            ~TileOrder() { on = false; }
+        } order(tile_order[1], runs_fixed_cycles(1));
         lo->check_quirks();
         push_to_shadow(start, {GLIDE_BED, GLIDE_B, GLIDE_BETA, GLIDE_SMB}, true, s);
         push_to_shadow(start, {GLIDE_U, GLIDE_V, GLIDE_H, GLIDE_H_PREV, GLIDE_PHI, GLIDE_MASK}, false, s);
@@ -1077,22 +1094,30 @@ struct Solver : SolverBase {
     void lin_op(int l, double dt, const Lin& L, const int* out, const int* sub, bool use_forcing, bool norms,
                 bool ref_rows, cudaStream_t s, int jvp_flags = GLIDE_USE_MASK) {
         StripArgs<R> q = strip_args(l, dt, L, out, sub, use_forcing, norms, ref_rows, jvp_flags);
-        if constexpr (sizeof(R) == 4) {
-            if (L.tr && fixed_cycles) {
-                const int fl[AdjTile<R>::NB] = {GLIDE_U, GLIDE_V, GLIDE_H, GLIDE_PHI, GLIDE_BED, GLIDE_BETA,
-                                                GLIDE_B, L.x[0], L.x[1]};
-                not_recordable("the tiled transposed product");
-                q.a.err = err_dev;
-                k_vjp<R><<<dim3(lv[l].blocks_x(), lv[l].blocks_y()), kTile * kTile, 0, s>>>(
-                    q.a, box_maps(l, fl, AdjTile<R>::BH));
-                counted("vjp", lb(l, 11 + (use_forcing ? 3 : 0) + (sub ? 3 : 0) + 3));
-                return;
-            }
-        }
-        const dim3 g = strip_grid<false>(q);
         // u, v, H, phi, mask, bed, beta, B and the three unknowns read, the
         // forcing and the subtrahend when given, three rows written
         const double bytes = lb(l, 11 + (use_forcing ? 3 : 0) + (sub ? 3 : 0) + 3);
+        if (tile_order[L.cfg]) {
+            not_recordable("a tiled product");
+            const dim3 g(lv[l].blocks_x(), lv[l].blocks_y());
+            q.a.err = err_dev;
+            if (L.tr) {
+                const int fl[AdjTile<R>::NB] = {GLIDE_U, GLIDE_V, GLIDE_H, GLIDE_PHI, GLIDE_BED, GLIDE_BETA,
+                                                GLIDE_B, L.x[0], L.x[1]};
+                k_vjp<R><<<g, kTile * kTile, 0, s>>>(q.a, box_maps(l, fl, AdjTile<R>::BH));
+            } else if constexpr (sizeof(R) == 4) {
+                const int fl[JvpTile<R>::NB] = {GLIDE_U, GLIDE_V, L.x[0], L.x[1], GLIDE_H, GLIDE_PHI, GLIDE_BED,
+                                                GLIDE_BETA, GLIDE_B, L.x[2]};
+                if (norms || ref_rows || q.mode) fail(GLIDE_ERR_STATE, "the tiled tangent product is the solver's own");
+                k_jvp<R><<<g, kTile * kTile, 0, s>>>(q.a, box_maps(l, fl, kBoxH));
+            } else {
+                fail(GLIDE_ERR_STATE, "tangent systems are solved on the binary32 half");
+            }
+            counted(L.tr ? "vjp" : "jvp", bytes);
+            if (norms) finish_norms(int(g.x * g.y), s);
+            return;
+        }
+        const dim3 g = strip_grid<false>(q);
         if (!record(G_LINEAR, L.tr ? 1 : 0, g, q, bytes)) {
             if (L.tr) k_linear_strip<R, true, false><<<g, 32 * kStripWarps, 0, s>>>(q);
             else k_linear_strip<R, false, false><<<g, 32 * kStripWarps, 0, s>>>(q);
@@ -1166,11 +1191,11 @@ struct Solver : SolverBase {
         if (factor) block_factor(l, dt, L, s);
         if (blk.empty()) fail(GLIDE_ERR_STATE, "block factor buffers not allocated");
         Level<R>& v = lv[l];
-        if (L.tr && fixed_cycles) {  // (adjoint_tile.cuh)
+        if (tile_order[L.cfg]) {
             const BlockArgs<R> a = block_args(l, dt, L);
             for (int k = 0; k < n; ++k) {
                 lin_residual(l, dt, L, false, s);
-                block_sweep(l, a, true, dim3(v.blocks_x(), v.blocks_y()), s);
+                block_sweep(l, a, L.tr, dim3(v.blocks_x(), v.blocks_y()), s);
             }
             return;
         }
