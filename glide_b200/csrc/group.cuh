@@ -33,8 +33,8 @@ namespace glide {
 // Launch kinds a hierarchy records for grouped execution.
 enum GroupOpKind {
     G_SNAPSHOT, G_RESTRICT, G_RESTRICT_BATCH, G_CORRECT_BATCH, G_GROUNDED, G_COPY, G_SET_RHS, G_SWEEP,
-    G_RESIDUAL, G_NORMS, G_LINEAR, G_SMOOTH, G_BLOCK_FACTOR, G_GRADIENTS, G_FILL, G_TANGENT_RHS, G_NEWTON_UPDATE,
-    G_KINDS
+    G_RESIDUAL, G_NORMS, G_LINEAR, G_SMOOTH, G_BLOCK_FACTOR, G_BLOCK_SWEEP, G_GRADIENTS, G_FILL, G_TANGENT_RHS,
+    G_NEWTON_UPDATE, G_KINDS
 };
 
 struct NormsArgs {
@@ -253,6 +253,15 @@ struct GBlockFactor {
     static constexpr int kThreads = kTile * kTile;
     static __device__ __forceinline__ void run(const Args& a, const unsigned char* mp, GroupBlock b) {
         block_factor_tile<R, TR>(a, item_maps<7>(mp), b);
+    }
+};
+template <class R, bool TR>
+struct GBlockSweep {
+    static constexpr int kMinBlocks = sizeof(R) == 8 ? 4 : 5;
+    using Args = BlockArgs<R>;
+    static constexpr int kThreads = kSweepThreads;
+    static __device__ __forceinline__ void run(const Args& a, const unsigned char*, GroupBlock b) {
+        block_sweep_tile<R, TR>(a, b);
     }
 };
 // The item holding tile t: the last item whose range starts at or before t.

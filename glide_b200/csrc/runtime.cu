@@ -1183,38 +1183,31 @@ struct Solver : SolverBase {
         counted("block_factor", bytes);
     }
 
-    // n linear smoother sweeps (residual, block solve and update in one pass,
-    // alternating between the unknowns' home and second buffers, ending at
-    // home); the factors are refreshed first unless the caller just did
+    // n linear smoother sweeps.  Two at a time they run as fused passes
+    // (residual, block solve and update) from the unknowns' home buffers into
+    // the second ones and back.  The last of an odd count has no way back: it is
+    // a residual pass and a block solve in place, which costs less than three
+    // copies before a fused one (with its factors, one sweep of 250^2 in binary64
+    // 40.0 -> 27.9 us, of 64^2 27.7 -> 21.4; of 2048^2 785 -> 751).  The factors
+    // are refreshed first unless the caller just did.
     void lin_sweeps(int l, double dt, int n, const Lin& L, cudaStream_t s, bool factor = true) {
         if (n <= 0) return;
         if (factor) block_factor(l, dt, L, s);
         if (blk.empty()) fail(GLIDE_ERR_STATE, "block factor buffers not allocated");
         Level<R>& v = lv[l];
-        if (tile_order[L.cfg]) {
-            const BlockArgs<R> a = block_args(l, dt, L);
-            for (int k = 0; k < n; ++k) {
-                lin_residual(l, dt, L, false, s);
-                block_sweep(l, a, L.tr, dim3(v.blocks_x(), v.blocks_y()), s);
-            }
-            return;
-        }
+        const int fused = tile_order[L.cfg] ? 0 : n - (n & 1);
         const int alt[3] = {F_XA_U, F_XA_V, F_XA_H};
         StripArgs<R> q = strip_args(l, dt, L, nullptr, nullptr, true, false, false, GLIDE_USE_MASK);
         q.fac = blk[l];
         q.plane = size_t(v.ny) * v.pc;
         q.omega = R(v.vk[L.cfg].omega);
         const dim3 g = strip_grid<true>(q);
-        const int start_alt = n & 1;
-        if (start_alt)
-            for (int k = 0; k < 3; ++k) copy(v.a[alt[k]], v.a[L.x[k]], s);
         // u, v, H, phi, mask, bed, beta, B, the unknowns and the forcing read, the
         // factors read, the unknowns written
         const double bytes = lb(l, 8 + 3 + 3 + 3) + factor_bytes(l, L.tr);
-        for (int k = 0; k < n; ++k) {
-            const bool in_alt = (start_alt ^ (k & 1)) != 0;
-            const int* in = in_alt ? alt : L.x;
-            const int* out = in_alt ? L.x : alt;
+        for (int k = 0; k < fused; ++k) {
+            const int* in = (k & 1) ? alt : L.x;
+            const int* out = (k & 1) ? L.x : alt;
             q.a.lu = v.a[in[0]]; q.a.lv = v.a[in[1]]; q.a.lH = v.a[in[2]];
             q.xu = v.a[out[0]]; q.xv = v.a[out[1]]; q.xH = v.a[out[2]];
             if (keep_residual && k == n - 1) {
@@ -1224,6 +1217,12 @@ struct Solver : SolverBase {
             if (L.tr) k_linear_strip<R, true, true><<<g, 32 * kStripWarps, 0, s>>>(q);
             else k_linear_strip<R, false, true><<<g, 32 * kStripWarps, 0, s>>>(q);
             counted("linear_sweep", bytes);
+        }
+        if (fused == n) return;
+        const BlockArgs<R> a = block_args(l, dt, L);
+        for (int k = fused; k < n; ++k) {
+            lin_residual(l, dt, L, false, s);
+            block_sweep(l, a, L.tr, dim3(v.blocks_x(), v.blocks_y()), s);
         }
     }
 
@@ -1246,7 +1245,7 @@ struct Solver : SolverBase {
     // 25 factors, r, x read; x written
     void block_sweep(int l, const BlockArgs<R>& a, bool tr, dim3 g, cudaStream_t s) {
         const double bytes = lb(l, 9) + factor_bytes(l, tr);
-        not_recordable("a block sweep alone");
+        if (record(G_BLOCK_SWEEP, tr ? 1 : 0, g, a, bytes)) return;
         if (tr) k_block_sweep<R, true><<<g, kSweepThreads, 0, s>>>(a);
         else k_block_sweep<R, false><<<g, kSweepThreads, 0, s>>>(a);
         counted("linear_sweep", bytes);
@@ -1691,6 +1690,8 @@ struct GroupRun : GroupBase {
             }
             case G_BLOCK_FACTOR:
                 return v ? issue_op<GBlockFactor<R, true>>(L, s) : issue_op<GBlockFactor<R, false>>(L, s);
+            case G_BLOCK_SWEEP:
+                return v ? issue_op<GBlockSweep<R, true>>(L, s) : issue_op<GBlockSweep<R, false>>(L, s);
             default: fail(GLIDE_ERR_STATE, "unknown grouped launch kind");
         }
         return 0;

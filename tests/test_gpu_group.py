@@ -173,3 +173,40 @@ def test_group_reports_a_nonfinite_member_and_solves_the_others():
     st = g.forward(DT)
     assert all(np.isfinite(s["final_norm"]) for s in st)
     g.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_odd_sweep_counts_in_a_group(precision):
+    """An odd count of linear sweeps ends in a residual pass and a block solve in place: their grouped launches, tangent
+    and adjoint, against the members' own solves of three cycles (bars as above)."""
+    from glide_b200.ensemble import CANDIDATES, apply_schedule
+    from glide_b200.group import HierarchyGroup
+    odd = dict(pre_steps=1, post_steps=3, finest_steps=1, coarsest_steps=5)
+
+    def members():
+        out = _members(precision)[:3]
+        for m in out:
+            apply_schedule(m, CANDIDATES["fast"])
+            for which in (False, True, 2):
+                m.mg.hierarchy.set_fas(which, **odd)
+            for s in (m.forward_solver, m.adjoint_solver):
+                s.fas_options.set(maximum_vcycles=3, relative_tolerance=0.0, absolute_tolerance=0.0)
+        return out
+
+    solo, grouped = members(), members()
+    for m in solo:
+        m.forward(0.0, DT, update_geometry=False)
+        du, dv, _ = _dJ(m)
+        m.backward(0.0, DT, dJdu=du, dJdv=dv)
+    g = HierarchyGroup([m.mg.hierarchy for m in grouped])
+    g.forward(DT)
+    masks = {m.prepare_backward(*_dJ(m)) for m in grouped}
+    g.backward(DT, mask=masks.pop())
+    torch.cuda.synchronize()
+    tol = 1e-10 if precision == "fp64" else 1e-3
+    for a, b in zip(solo, grouped):
+        for k in ("u", "v", "H", "lambda_u", "lambda_v", "lambda_H", "grad_beta"):
+            x = a.mg.hierarchy.get(k, 0).double().cpu().numpy()
+            y = b.mg.hierarchy.get(k, 0).double().cpu().numpy()
+            assert rel_err(y, x) <= tol, (k, rel_err(y, x))
+    g.close()

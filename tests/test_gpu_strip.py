@@ -58,7 +58,7 @@ def test_transposed_product_and_sweeps_match_oracle(ny, nx, phys):
     lev.adj_vjp(DT)
     for k in "uvH":
         assert rel_err(h.view("vjp_" + k, 0).cpu().numpy(), getattr(lev, "vjp_" + k)) <= 1e-12, k
-    for n in (3, 2):  # an odd count starts in the second buffer
+    for n in (3, 2, 1):  # fused in pairs; the last of an odd count is a product and a block solve
         h.adjoint_sweep(0, DT, n)
         lev.adj_sweep(DT, n)
         for k in "uvH":
