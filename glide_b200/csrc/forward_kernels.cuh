@@ -156,9 +156,9 @@ __global__ void k_grounded(Arr<R> phi, Arr<R> H, Arr<R> bed, R c, R relax, int n
 // the two cells sharing a face, and the omega-update -- written to a second
 // state buffer, because every cell reads its neighbours' old values.
 //
-// Block = 16x16 own cells + the 16 cells left of the tile + the 16 cells
-// above it (288 threads).  The halo cells are solved redundantly so that the
-// block owns its faces outright: no atomics, no zero fills, no separate axpy.
+// A block of BY x BX threads owns (BY - 1) x (BX - 1) cells.  The row above and
+// the column left of them are solved redundantly so that the block owns its
+// faces outright: no atomics, no zero fills, no separate axpy.
 // -------------------------------------------------------------------------
 enum GammaMode { kGammaArray = 0, kGammaWChi = 1, kGammaWPhi = 2 };
 

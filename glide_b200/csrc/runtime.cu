@@ -185,26 +185,57 @@ struct RecOp {
     std::vector<unsigned char> maps;  // the staging maps of a stencil launch (BoxMaps)
 };
 
-// The forms of the Vanka sweep a launch picks from: the general one at one of
-// two register budgets, or the linear-sliding one.
+// The forms of the Vanka sweep a launch picks from: the general one at the
+// register budget of one or two blocks per SM, in the latter case in one of three
+// shapes, or the linear-sliding one.
 //
 // Blocks of whole groups of four warps fill the four register files evenly
-// (288-thread blocks left a quarter of them idle).  Binary64, general: 8 x 16
-// threads (7 x 15 owned cells) at 3 per SM run a 3-V-cycle step of 512^2 / 64^2
-// in 53.2 / 27.8 ms, 16 x 16 at 2 per SM 54.1 / 34.8, 8 x 16 at 4 per SM 54.7 /
-// 32.3, 8 x 8 at 5 per SM 58.0 / 29.4; 288-thread blocks took 56.5 / 31.1.
+// (288-thread blocks left a quarter of them idle).  On small grids the sweep is
+// one latency chain, which the smaller blocks shorten; on large ones it is bound
+// by throughput and by how full the last wave is.
+//
+// Binary64 (eight sweeps of a dome; 288-thread blocks / 8 x 16 threads, 7 x 15
+// owned cells, at 3 per SM / at 4 / 16 x 16 at 2), m = 1/3: 64^2 1914 / 1323 /
+// 1414 / 1552 us, 192^2 1903 / 1703 / 1815 / 2160, 250^2 2747 / 3085 / 3145 /
+// 2140, 512^2 8934 / 9335 / 9234 / 8696, 2048^2 144 / 146 / 140 / 129 ms.  With
+// the 168 registers of 3 per SM the compiler contracts the power law's sums
+// otherwise, so that a cell's count of local iterations flips at its threshold now
+// and then (up to 2e-2 in that cell's H on a rough state); the others agree with
+// the 288-thread form bit for bit.  So with m != 1: 8 x 16 at 4 per SM on up to one
+// wave of 3 per SM (444 blocks), then 16 x 16.  With m = 1 all agree; 8 x 16 at 3
+// per SM and 16 x 16 are within 5 % of each other from 320^2 on (512^2 3836 / 3849
+// us), and the first takes a 3-V-cycle step of 512^2 / 64^2 in 53.2 / 27.8 ms
+// (16 x 16 54.1 / 34.8, 8 x 16 at 4 per SM 54.7 / 32.3, 288 threads 56.5 / 31.1).
+//
+// Binary32, general, 288-thread / 8 x 16 at 5 per SM / 10 x 32 (9 x 31 cells) at
+// 2: m = 1/3 64^2 469 / 340 / 453 us, 128^2 468 / 387 / 452, 512^2 1949 / 2017 /
+// 2001, 768^2 4382 / 4457 / 4328, 2048^2 30.2 / 30.7 / 29.5 ms; a V-cycle of a
+// mixed handle 64^2 6.09 / 5.14 / 6.38 ms, 512^2 19.9 / 19.3 / 20.2, 1024^2 68.9 /
+// 68.7 / 69.4.  So the wide blocks from four waves of the small ones on (4 x 740).
+//
 // Binary32, linear (600 x 424, 2 V-cycles): 8 x 16 at 5 per SM 9.36 ms, at 3 or
 // 4 per SM 9.74.
-enum SweepFormId { S_GENERAL_1, S_GENERAL_2, S_LINEAR };
+enum SweepFormId { S_GENERAL_1, S_GENERAL_2, S_GENERAL_POW, S_GENERAL_WIDE, S_LINEAR };
 template <class R, class F>
 static void with_sweep_form(int form, F&& f) {
     constexpr bool wide = sizeof(R) == 8;
     switch (form) {
         case S_GENERAL_1: f(SweepForm<false, wide ? 8 : 16, 16, wide ? 2 : 1>{}); break;
-        case S_GENERAL_2: f(SweepForm<false, wide ? 8 : 16, 16, wide ? 3 : 2>{}); break;
+        case S_GENERAL_2: f(SweepForm<false, 8, 16, wide ? 3 : 5>{}); break;
+        case S_GENERAL_POW: f(SweepForm<false, 8, 16, wide ? 4 : 5>{}); break;
+        case S_GENERAL_WIDE: f(SweepForm<false, wide ? 16 : 10, wide ? 16 : 32, 2>{}); break;
         case S_LINEAR: f(SweepForm<!wide, 8, 16, wide ? 3 : 5>{}); break;
         default: fail(GLIDE_ERR_STATE, "unknown sweep form");
     }
+}
+
+// the block shape of the general form at two blocks per SM (figures above)
+template <class R>
+static int general_sweep_form(int ny, int nx, bool linear_sliding) {
+    const long long blocks = (long long)((nx + 14) / 15) * ((ny + 6) / 7);
+    if (sizeof(R) == 8)
+        return linear_sliding ? S_GENERAL_2 : blocks > 148 * 3 ? S_GENERAL_WIDE : S_GENERAL_POW;
+    return blocks > 4 * 148 * 5 ? S_GENERAL_WIDE : S_GENERAL_2;
 }
 
 template <class R>
@@ -624,13 +655,17 @@ struct Solver : SolverBase {
     void launch_sweep(const SweepArgs<R>& a, bool phi_live, cudaStream_t s, double bytes) {
         // The linear-sliding form reorders the local system's sums and divides
         // by diagonals of at least damping + drag (local_cell.cuh).  It runs on
-        // binary32 handles only.  Binary64 and mixed handles promise the
-        // reference's binary64 iterates: there the local iteration stops on a
-        // threshold at which a reordered sum flips a cell's count now and then
-        // (2 of 26 adjoint runs at 512^2, up to 4e-9 in the gradients), and a
-        // fixed number of mixed cycles carries its shadow's rounding (6e-6).
+        // binary32 handles only.  In solves of a fixed number of cycles binary64
+        // and mixed handles keep the iterates of the reference's order: the local
+        // iteration stops on a threshold at which a reordered sum flips a cell's
+        // count now and then (2 of 26 adjoint runs at 512^2, up to 4e-9 in the
+        // gradients), and a mixed iterate carries its binary32 half's rounding
+        // (6e-6).  Solves of those handles to a tolerance could take it; they
+        // have not been measured with it.
         const bool linear = sizeof(R) == 4 && !shadow && a.p.m == R(1) && a.ssa_damping + a.p.water_drag > R(0);
-        const int form = linear ? S_LINEAR : (sweep_blocks_per_sm >= 2 ? S_GENERAL_2 : S_GENERAL_1);
+        const int form = linear ? S_LINEAR
+                                : sweep_blocks_per_sm < 2 ? S_GENERAL_1
+                                                          : general_sweep_form<R>(a.ny, a.nx, a.p.m == R(1));
         with_sweep_form<R>(form, [&](auto f) {
             launch_sweep_form<decltype(f)>(a, phi_live, (phi_live ? 1 : 0) | 2 * form, s, bytes);
         });

@@ -1,14 +1,15 @@
-"""The Vanka sweep's linear-sliding form (glide_b200/csrc/local_cell.cuh) and
-its general form against the oracle's sweeps, at the edges of the blocks' 7 x 15
-owned cells and on the smallest levels.
+"""The Vanka sweep's forms against the oracle's sweeps in binary64, at the edges of
+their blocks and on the smallest levels: the linear-sliding local iteration
+(glide_b200/csrc/local_cell.cuh: m = 1, damping + drag > 0, binary32) and the
+general one, whose block shape depends on the size, the precision and m.
 
-binary64: 1e-10, the multi-sweep parity bar.  binary32: 2e-4, the bar of the
-binary32 solves, for all but a few values: a cell whose H - dt r_H lies within
-binary32 rounding of gamma may take the other active-set decision.  With
-|H - dt r_H| up to 1e5 spread over about 1e3 that is 6e-6 of the decisions, 60
-of them per cell in two sweeps -- about one cell at the largest size here --
-and one such cell reaches the 5 x 5 around it in the two sweeps: two cells' worth,
-50 values, may differ.
+The inputs are binary32 numbers, so both sides solve the same cells.  Velocities of
+5 m/a keep |H - dt r_H - gamma| above the binary32 rounding of its terms (1e-4 m)
+in every cell used here, so no active-set decision may differ and no value is
+excused.  Bars: binary64 1e-10, the multi-sweep parity bar.  Binary32, of the
+largest value: one sweep ends within a few roundings of the local solution
+(measured 3e-7 linear, 6e-7 general: 2e-6 and 4e-6); the second starts from that
+and multiplies it by the local conditioning (2e-6, 1.2e-5: 1e-5 and 5e-5).
 """
 from __future__ import annotations
 
@@ -16,49 +17,86 @@ import numpy as np
 import pytest
 
 from cases import random_state
-from util import oracle_single_level, rel_err
+from util import oracle_single_level
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 DX, DT = 1500.0, 5.0
-SIZES = [(2, 2), (7, 15), (8, 16), (6, 14), (15, 31), (22, 9), (33, 61)]
+SIZES = [(2, 2), (3, 2), (2, 40), (7, 15), (8, 16), (6, 14), (15, 31), (22, 9), (33, 61), (120, 150)]
+LINEAR_BAR = {1: 2e-6, 2: 1e-5}
+GENERAL_BAR = {1: 4e-6, 2: 5e-5}
 
 
-def _run(ny, nx, dtype, phys=None, sweeps=2):
+def _state(ny, nx, thin=0.0):
+    f = random_state(ny, nx, seed=100 * ny + nx, thin_frac=thin)
+    f["u"], f["v"] = 0.1 * f["u"], 0.1 * f["v"]
+    return {k: np.asarray(a, np.float32).astype(np.float64) for k, a in f.items()}
+
+
+def _sweep(f, dtype, phys, sweeps):
     from glide_b200.hierarchy import Hierarchy
-    f = random_state(ny, nx, seed=100 * ny + nx)
-    h = Hierarchy(ny, nx, DX, 1, dtype=torch.float64 if dtype == np.float64 else torch.float32)
+    h = Hierarchy(*f["H"].shape, DX, 1, dtype=dtype)
     for k in ("u", "v", "H", "H_prev", "mask", "bed", "B", "beta", "smb", "f_u", "f_v"):
         h.set(k, 0, torch.as_tensor(f[k]))
-    o = oracle_single_level({f"in_{k}": a for k, a in f.items()}, DX, dtype=dtype)
-    lev = o.levels[0]
-    if phys:
-        h.set_phys(-1, **phys)
-        o.set_phys(**phys)
+    h.set_phys(-1, **phys)
     h.set_rhs(0, DT)
-    lev.f_H[...] = lev.H_prev / dtype(DT) + lev.smb
     h.vanka_sweep(0, DT, sweeps)
+    return {k: h.get(k, 0).cpu().numpy() for k in ("u", "v", "H", "mask")}
+
+
+def _check(f, dtype, phys, sweeps, bar):
+    got = _sweep(f, dtype, phys, sweeps)
+    o = oracle_single_level({f"in_{k}": a for k, a in f.items()}, DX)
+    o.set_phys(**phys)
+    lev = o.levels[0]
+    lev.f_H[...] = lev.H_prev / DT + lev.smb
     lev.vanka_sweep(DT, sweeps)
-    return {k: (h.view(k, 0).cpu().numpy(), getattr(lev, k)) for k in ("u", "v", "H", "mask")}
-
-
-@pytest.mark.parametrize("dtype,tol", [(np.float64, 1e-10), (np.float32, 2e-4)])
-@pytest.mark.parametrize("ny,nx", SIZES)
-def test_linear_sliding_sweeps_match_oracle(ny, nx, dtype, tol):
-    got = _run(ny, nx, dtype, phys=dict(calving_rate=2.0))
     for k in ("u", "v", "H"):
-        a, b = got[k]
-        off = np.abs(a - b) > tol * np.abs(b).max()
-        assert off.sum() <= (0 if dtype == np.float64 else 50), k
-    if dtype == np.float64:
-        assert (got["mask"][0] == got["mask"][1]).mean() >= 0.998
+        want = getattr(lev, k)
+        assert np.isfinite(got[k]).all(), k
+        assert np.abs(got[k] - want).max() <= bar * np.abs(want).max(), (k, np.abs(got[k] - want).max())
+    np.testing.assert_array_equal(got["mask"], lev.mask)
 
 
-@pytest.mark.parametrize("phys", [dict(m=1.0 / 3.0), dict(water_drag=-0.02)])
-def test_general_form_matches_oracle(phys):
-    """Nonlinear sliding, or a drag that leaves the diagonals unbounded below, runs the general form."""
-    for ny, nx in ((8, 16), (31, 16)):
-        got = _run(ny, nx, np.float64, phys=phys)
-        for k in ("u", "v", "H"):
-            assert rel_err(*got[k]) <= 1e-10, (k, ny, nx)
+@pytest.mark.parametrize("sweeps,thin", [(1, 0.0), (1, 0.2), (2, 0.0)])
+@pytest.mark.parametrize("ny,nx", SIZES)
+def test_linear_sliding_in_binary32(ny, nx, sweeps, thin):
+    _check(_state(ny, nx, thin), torch.float32, dict(calving_rate=2.0), sweeps, LINEAR_BAR[sweeps])
+
+
+@pytest.mark.parametrize("phys", [dict(calving_rate=2.0), dict(m=1.0 / 3.0), dict(water_drag=-0.02)])
+@pytest.mark.parametrize("ny,nx", SIZES)
+def test_general_form_in_binary64(ny, nx, phys):
+    # thin cells have nothing but the drag on their diagonals, and a negative one makes some nearly singular
+    _check(_state(ny, nx, 0.0 if "water_drag" in phys else 0.2), torch.float64, phys, 2, 1e-10)
+
+
+@pytest.mark.parametrize("phys", [dict(m=1.0 / 3.0), dict(water_drag=-0.02), dict(m=1.0 + 2.0 ** -22)])
+@pytest.mark.parametrize("ny,nx", SIZES)
+def test_general_form_in_binary32(ny, nx, phys):
+    """Nonlinear sliding (as little as one step from m = 1: the linear form ignores the power law), or a drag that
+    leaves the diagonals unbounded, is solved by the general form."""
+    for sweeps in (1, 2):
+        _check(_state(ny, nx), torch.float32, phys, sweeps, GENERAL_BAR[sweeps])
+
+
+@pytest.mark.parametrize("dtype,ny,nx", [(torch.float64, 224, 226), (torch.float32, 378, 826)])
+def test_wide_blocks_match_oracle(dtype, ny, nx):
+    """Just above the sizes where the general form takes its larger blocks (444 and 2960 small ones), ragged in both
+    directions."""
+    bar = 1e-10 if dtype == torch.float64 else GENERAL_BAR[1]
+    _check(_state(ny, nx), dtype, dict(m=1.0 / 3.0), 1, bar)
+
+
+@pytest.mark.parametrize("dtype,small,large", [(torch.float64, (120, 150), (224, 226)),
+                                               (torch.float32, (300, 330), (378, 826))])
+def test_block_shape_changes_no_bit(dtype, small, large):
+    """Three sweeps of the upper left cells of a large grid and of a grid cut there agree bit for bit where the cut is
+    out of reach (three cells a sweep), on a rough state whose cells stop at every count of local iterations."""
+    f = random_state(*large, seed=5)
+    ny, nx = small
+    cut = {k: a[:ny + (k in ("v", "f_v")), :nx + (k in ("u", "f_u"))].copy() for k, a in f.items()}
+    a, b = (_sweep(s, dtype, dict(m=1.0 / 3.0), 3) for s in (f, cut))
+    for k in ("u", "v", "H", "mask"):
+        np.testing.assert_array_equal(a[k][:ny - 10, :nx - 10], b[k][:ny - 10, :nx - 10], err_msg=k)
