@@ -84,11 +84,10 @@ __device__ __forceinline__ double pow_small(double q, double e) {
     return fma(x, r_low, x) * __hiloint2double((int(n) + 1023) << 20, 0);
 }
 
-// Two powers of one exponent in one call.  Each pow() is a chain of some 150
-// dependent operations behind a call of its own; these two chains are shorter
-// and overlap.
+// Two powers of one exponent.  Each pow() is a chain of some 150 dependent
+// operations behind a call of its own; these two chains are shorter and overlap.
 struct PowPair { double a, b; };
-__device__ __noinline__ inline PowPair pow_pair(double x, double y, double e) {
+__device__ __forceinline__ PowPair pow_two(double x, double y, double e) {
     constexpr double lo = 1e-280, up = 1e280;  // 2^n stays a normal number
     if (fabs(e) <= 1.0 && x > lo && x < up && y > lo && y < up) return {pow_small(x, e), pow_small(y, e)};
     return {pow(x, e), pow(y, e)};
@@ -96,9 +95,22 @@ __device__ __noinline__ inline PowPair pow_pair(double x, double y, double e) {
 
 // d q^e / dq from the power itself.  At q = 0 the quotient says nothing (0 / 0
 // where the derivative is finite).
-__device__ __forceinline__ double pow_slope(double q, double pw, double e) {
-    return q > 0.0 ? e * pw / q : e * pow_general(q, e - 1.0);
+template <class P>
+__device__ __forceinline__ double pow_slope(double q, double pw, double e, P&& power) {
+    return q > 0.0 ? e * pw / q : e * power(q, e - 1.0);
 }
+
+// The powers of a row step's two faces with their derivatives, out of line so that
+// linear sliding keeps its registers: all four for the smoother (the derivatives in
+// line cost it 1 % with m = 1), the powers for the product, where a result that
+// comes back on the stack costs more (J e with m = 1 at 2048^2: 219 us, 273 so).
+struct SlidePair { double a, da, b, db; };
+__device__ __noinline__ inline SlidePair slide_pair(double x, double y, double e) {
+    const PowPair p = pow_two(x, y, e);
+    auto power = [](double q, double k) { return pow(q, k); };
+    return {p.a, pow_slope(x, p.a, e, power), p.b, pow_slope(y, p.b, e, power)};
+}
+__device__ __noinline__ inline PowPair pow_pair(double x, double y, double e) { return pow_two(x, y, e); }
 
 // The neighbouring lanes' values.  All 32 lanes must call: never inside a
 // conditional expression or a branch that is not uniform over the warp.
@@ -250,12 +262,18 @@ __device__ __forceinline__ void linear_strip(const StripArgs<R>& q, BLK blk) {
                     // at 64^2 (12.3).  J^T lambda 50 -> 33 at 512^2 (60).
                     hu = hv = 0;
                     if (TR || (t >= first && (SMOOTH || t < rb))) {
-                        const PowPair pw = pow_pair(qu, qv, e);
-                        const R dpu = pow_slope(qu, pw.a, e), dpv = pow_slope(qv, pw.b, e);
-                        ru -= (beu * (R(2) * dpu * u0 * u0 + pw.a) + p.water_drag) * eu0;
-                        rv -= (bev * (R(2) * dpv * v0 * v0 + pw.b) + p.water_drag) * ev0;
-                        hu = -beu * (R(0.5) * dpu * u0);
-                        hv = -bev * (R(0.5) * dpv * v0);
+                        SlidePair w;
+                        if constexpr (SMOOTH) {
+                            w = slide_pair(qu, qv, e);
+                        } else {
+                            const PowPair pw = pow_pair(qu, qv, e);
+                            w = {pw.a, pow_slope(qu, pw.a, e, pow_general<double>), pw.b,
+                                 pow_slope(qv, pw.b, e, pow_general<double>)};
+                        }
+                        ru -= (beu * (R(2) * w.da * u0 * u0 + w.a) + p.water_drag) * eu0;
+                        rv -= (bev * (R(2) * w.db * v0 * v0 + w.b) + p.water_drag) * ev0;
+                        hu = -beu * (R(0.5) * w.da * u0);
+                        hv = -bev * (R(0.5) * w.db * v0);
                     }
                 } else {
                     const R dpu = e * pow_general(qu, e - R(1)), dpv = e * pow_general(qv, e - R(1));
