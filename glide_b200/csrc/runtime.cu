@@ -202,16 +202,25 @@ struct RecOp {
 // otherwise, so that a cell's count of local iterations flips at its threshold now
 // and then (up to 2e-2 in that cell's H on a rough state); the others agree with
 // the 288-thread form bit for bit.  So with m != 1: 8 x 16 at 4 per SM on up to one
-// wave of 3 per SM (444 blocks), then 16 x 16.  With m = 1 all agree; 8 x 16 at 3
-// per SM and 16 x 16 are within 5 % of each other from 320^2 on (512^2 3836 / 3849
-// us), and the first takes a 3-V-cycle step of 512^2 / 64^2 in 53.2 / 27.8 ms
-// (16 x 16 54.1 / 34.8, 8 x 16 at 4 per SM 54.7 / 32.3, 288 threads 56.5 / 31.1).
+// wave of 3 per SM (444 blocks), then 16 x 16.
+//
+// With m = 1 all agree, and what counts is how many blocks the fullest SM gets:
+// eight sweeps take about 55 us plus 645 for every three 8 x 16 blocks on it (one
+// left over 350, two 560), or 75 plus 855 for every two 16 x 16 blocks (one left
+// over 520): 240^2 1093 / 930 us, 256^2 1212 / 1445, 400^2 2428 / 2267, 704^2 6931
+// / 6413.  The estimate picks, 16 x 16 within 3 %: its 128 registers leave room
+// beside other streams' kernels, which an ensemble's members run (64 mixed
+// members on 16 streams, whose fallback cycles are binary64: 7.05 s a step with 8
+// x 16 alone, 6.06 so, 6.80 with 288 threads).  A 3-V-cycle step of 512^2 / 64^2
+// takes 51.6 / 27.7 ms (288 threads 56.5 / 31.1, 8 x 16 alone 53.2 / 27.7).
 //
 // Binary32, general, 288-thread / 8 x 16 at 5 per SM / 10 x 32 (9 x 31 cells) at
 // 2: m = 1/3 64^2 469 / 340 / 453 us, 128^2 468 / 387 / 452, 512^2 1949 / 2017 /
 // 2001, 768^2 4382 / 4457 / 4328, 2048^2 30.2 / 30.7 / 29.5 ms; a V-cycle of a
 // mixed handle 64^2 6.09 / 5.14 / 6.38 ms, 512^2 19.9 / 19.3 / 20.2, 1024^2 68.9 /
 // 68.7 / 69.4.  So the wide blocks from four waves of the small ones on (4 x 740).
+// In between, one level's sweeps go either way with how the last wave fills (208^2
+// 630 / 464, 272^2 639 / 771, 368^2 1160 / 1146, 480^2 1915 / 1766 us).
 //
 // Binary32, linear (600 x 424, 2 V-cycles): 8 x 16 at 5 per SM 9.36 ms, at 3 or
 // 4 per SM 9.74.
@@ -229,13 +238,19 @@ static void with_sweep_form(int form, F&& f) {
     }
 }
 
-// the block shape of the general form at two blocks per SM (figures above)
+// the shape of the general form at two blocks per SM (figures above)
 template <class R>
 static int general_sweep_form(int ny, int nx, bool linear_sliding) {
-    const long long blocks = (long long)((nx + 14) / 15) * ((ny + 6) / 7);
-    if (sizeof(R) == 8)
-        return linear_sliding ? S_GENERAL_2 : blocks > 148 * 3 ? S_GENERAL_WIDE : S_GENERAL_POW;
-    return blocks > 4 * 148 * 5 ? S_GENERAL_WIDE : S_GENERAL_2;
+    constexpr int sms = 148;
+    const long long small = (long long)((nx + 14) / 15) * ((ny + 6) / 7);
+    if (sizeof(R) == 4) return small > 4 * sms * 5 ? S_GENERAL_WIDE : S_GENERAL_2;
+    if (!linear_sliding) return small > 3 * sms ? S_GENERAL_WIDE : S_GENERAL_POW;
+    if (small <= 3 * sms) return S_GENERAL_2;
+    const long long wide = (long long)((nx + 14) / 15) * ((ny + 14) / 15);
+    const long long ks = (small + sms - 1) / sms, kw = (wide + sms - 1) / sms;  // blocks of the fullest SM
+    const double t_small = 55 + 645.0 * (ks / 3) + (ks % 3 == 1 ? 350 : ks % 3 == 2 ? 560 : 0);
+    const double t_wide = 75 + 855.0 * (kw / 2) + (kw % 2 ? 520 : 0);
+    return t_wide < 1.03 * t_small ? S_GENERAL_WIDE : S_GENERAL_2;
 }
 
 template <class R>
