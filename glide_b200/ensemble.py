@@ -8,10 +8,10 @@ calls release the interpreter lock, so the GPU runs kernels of many members
 at once.  A member's convergence checks synchronise only its own stream.
 
 `Ensemble.autotune` picks, per size class, the fastest of a few solver
-schedules and FASCD launch shapes (resident Vanka-sweep blocks per SM) by
-timing a step of the class's first member from a warm state: the member is
-first advanced one step, trials run from that state, and the member's
-original state is restored afterwards.
+schedules and FASCD launch shapes (resident Vanka-sweep blocks per SM) that
+converges for every member: it times a step of the class's first member from a
+warm state (the member advanced one step), tries the fastest on the others, and
+restores the members' original states afterwards.
 
 With `grouped=True` the members' cycles run in grouped launches
 (glide_b200.group): one forward solve and one adjoint solve cover the group
@@ -365,13 +365,31 @@ class Ensemble:
                 res[k] = s
         return res
 
+    def _warm(self, m: IceDynamics, dt: float, candidates: dict, original: dict) -> dict:
+        """The state one step on: solved from `original` under the first candidate, the others in turn if it stops
+        short; the next step starts from the solved geometry."""
+        h = m.mg.hierarchy
+        for name in list(candidates) + [FALLBACK]:
+            for f, v in original.items():
+                h.set(f, 0, v, restrict_down=True)
+            apply_schedule(m, candidates.get(name, CANDIDATES[FALLBACK]))
+            if _converged(m, m.forward(0.0, dt, update_geometry=False)):
+                break
+        saved = {f: h.get(f, 0) for f in STATE}
+        saved["H_prev"] = saved["H"].clone()
+        return saved
+
     def autotune(self, dt: float, candidates: dict | None = None, warm: bool = True) -> dict[int, str]:
         """Per size class: time one forward step of the class's first member
         with every candidate schedule, keep the fastest that converges for the
-        whole class.  With `warm`, the member is first advanced one step (the
-        "fast" schedule, the others in turn if it stops short), so the trials
-        time the warm-started steps a run is made of rather than its cold
-        first step; every trial starts from that state and the member's
+        whole class: the candidates that converge for the first member are
+        tried on the others, fastest first, until one converges for all; if
+        none does, the one that stops short for the fewest.  (A member that
+        stops short pays a second solve in its step, several times the
+        difference between two candidates.)  With `warm`, the members are first
+        advanced one step (the "fast" schedule, the others in turn if it stops short), so the trials
+        see the warm-started steps a run is made of rather than the cold
+        first step; every trial starts from that state and the members'
         original state is restored at the end."""
         candidates = candidates or CANDIDATES
         classes: dict[int, list[int]] = {}
@@ -381,43 +399,49 @@ class Ensemble:
         for n, ks in sorted(classes.items()):
             m = self.members[ks[0]]
             h = m.mg.hierarchy
-            original = {f: h.get(f, 0) for f in STATE}
-            saved = original
-            if warm:
-                for name in list(candidates) + [FALLBACK]:
-                    for f, v in original.items():
-                        h.set(f, 0, v, restrict_down=True)
-                    apply_schedule(m, candidates.get(name, CANDIDATES[FALLBACK]))
-                    st = m.forward(0.0, dt, update_geometry=False)
-                    if _converged(m, st):
-                        break
-                saved = {f: h.get(f, 0) for f in STATE}
-                saved["H_prev"] = saved["H"].clone()  # the next step starts from the solved geometry
-            best, best_t = None, float("inf")
+            original = {k: {f: self.members[k].mg.hierarchy.get(f, 0) for f in STATE} for k in ks}
+            saved = {ks[0]: self._warm(m, dt, candidates, original[ks[0]]) if warm else original[ks[0]]}
+            trials = self.trials.setdefault(n, {})
             for name, cfg in candidates.items():
                 apply_schedule(m, cfg)
                 for trial in range(2):  # the first run captures the V-cycle graphs
-                    for f, v in saved.items():
+                    for f, v in saved[ks[0]].items():
                         h.set(f, 0, v, restrict_down=True)
                     torch.cuda.synchronize()
                     t0 = time.perf_counter()
                     st = m.forward(0.0, dt, update_geometry=False)
                     torch.cuda.synchronize()
                     el = time.perf_counter() - t0
-                ok = st["final_norm"] <= max(h.get_fas(False)["relative_tolerance"] * st["initial_norm"],
-                                             h.get_fas(False)["absolute_tolerance"])
                 h0 = st["history"][0] if st["history"] and st["history"][0] > 0 else 1.0
-                self.trials.setdefault(n, {})[name] = {
-                    "ms": el * 1e3, "vcycles": int(st["vcycles"]), "converged": bool(ok),
-                    "history": [float(f"{x / h0:.2e}") for x in st["history"][:12]]}
-                if ok and el < best_t:
-                    best, best_t = name, el
-            best = best or FALLBACK
-            for f, v in original.items():
-                h.set(f, 0, v, restrict_down=True)
+                trials[name] = {"ms": el * 1e3, "vcycles": int(st["vcycles"]), "converged": _converged(m, st),
+                                "history": [float(f"{x / h0:.2e}") for x in st["history"][:12]]}
+            ranked = sorted((t["ms"], name) for name, t in trials.items() if name in candidates and t["converged"])
+            others = ks[1:]
+            if others and len(ranked) > 1:
+                def warm_up(k, mk):
+                    saved[k] = self._warm(mk, dt, candidates, original[k]) if warm else original[k]
+                self._run(warm_up, keys=others)
+            best, fewest = FALLBACK, len(ks) + 1
+            for _, name in ranked:
+                short = 0
+                if others and len(ranked) > 1:
+                    def solve(k, mk):
+                        for f, v in saved[k].items():
+                            mk.mg.hierarchy.set(f, 0, v, restrict_down=True)
+                        apply_schedule(mk, candidates[name])
+                        return _converged(mk, mk.forward(0.0, dt, update_geometry=False))
+                    res, _ = self._run(solve, keys=others)
+                    short = sum(not res[k] for k in others)
+                    trials[name]["members_short"] = short
+                if short < fewest:
+                    best, fewest = name, short
+                if short == 0:
+                    break
             for k in ks:
-                apply_schedule(self.members[k], candidates[best])
+                hk = self.members[k].mg.hierarchy
+                for f, v in original[k].items():
+                    hk.set(f, 0, v, restrict_down=True)
+                apply_schedule(self.members[k], candidates.get(best, CANDIDATES[FALLBACK]))
                 self.schedules[k] = best
             chosen[n] = best
         return chosen
-

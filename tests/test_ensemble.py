@@ -45,6 +45,51 @@ def _member(n, seed, levels=3, dx=4000.0):
     return m
 
 
+class _FakeMember:
+    """A member whose solves take as long as, and converge under, the schedules it is told."""
+
+    def __init__(self, n, cost, converges):
+        from types import SimpleNamespace
+        self.cost, self.converges, self.name = cost, converges, None
+        fields = {}
+        hier = SimpleNamespace(shapes=[(n, n, 0)], get=lambda f, level: fields.get(f, torch.zeros(1)).clone(),
+                               set=lambda f, level, v, restrict_down=False: fields.__setitem__(f, v.clone()),
+                               get_fas=lambda adjoint: dict(relative_tolerance=1e-8, absolute_tolerance=0.0))
+        self.fields, self.mg = fields, SimpleNamespace(hierarchy=hier)
+        self.forward_solver = SimpleNamespace(_fas_config=SimpleNamespace(relative_tolerance=1e-8,
+                                                                          absolute_tolerance=0.0))
+
+    def forward(self, t, dt, update_geometry=True):
+        import time
+        time.sleep(self.cost[self.name])
+        self.fields["H"] = self.mg.hierarchy.get("H", 0) + 1.0
+        final = 1e-9 if self.name in self.converges else 1e-3
+        return dict(initial_norm=1.0, final_norm=final, vcycles=1, history=[1.0, final])
+
+
+@pytest.mark.parametrize("others,want", [
+    ([{"a", "b", "c"}, {"a", "b", "c"}], "a"),   # the fastest converges for all
+    ([{"a", "b", "c"}, {"b", "c"}], "b"),        # ... not for the last member
+    ([{"b"}, {"c"}], "b"),                       # none does: the fastest of those that leave the fewest short
+])
+def test_autotune_keeps_what_converges_for_the_whole_class(monkeypatch, others, want):
+    from glide_b200 import ensemble
+    cost = {"a": 0.002, "b": 0.01, "c": 0.03}
+    members = [_FakeMember(64, cost, {"a", "b", "c"})] + [_FakeMember(64, cost, c) for c in others]
+    monkeypatch.setattr(ensemble, "apply_schedule", lambda m, cfg: setattr(m, "name", cfg["name"]))
+    monkeypatch.setattr(ensemble.torch.cuda, "synchronize", lambda: None)
+
+    class Serial(ensemble.Ensemble):
+        def _run(self, fn, keys=None, sides=()):
+            return [fn(k, m) if k in keys else None for k, m in enumerate(self.members)], []
+
+    ens = Serial(members, workers=1)
+    assert ens.autotune(1.0, candidates={k: dict(name=k) for k in cost}) == {64: want}
+    assert set(ens.schedules.values()) == {want} and all(m.name == want for m in members)
+    for m in members:  # as it was before the trials
+        assert float(m.mg.hierarchy.get("H", 0)) == 0.0
+
+
 @pytest.mark.gpu
 def test_concurrent_members_match_solo_runs():
     from glide_b200.ensemble import Ensemble
