@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(kColThreads, MINB) k_enth_column(EnthArgs a, d
     for (int it = 0; it < a.n_newton; ++it) {
         double Epk = e_pmp(0.0, x.h), Epp = e_pmp(dsig, x.h);
         double om_k = om[0];
-        Iface lo{0, 0, 0, 0, 0};
+    Iface lo{0, 0, 0, 0, 0};
         double c_prev = 0.0, d_prev = 0.0;
         // the iterate window of row k and the inputs of row k + 1 are
         // loaded before row k is assembled
@@ -526,7 +526,7 @@ __device__ __forceinline__ void column_newton_step(const EnthArgs& a, const Colu
     const double* src = FIRST ? E : El;
     double Epk = e_pmp(0.0, x.h), Epp = e_pmp(dsig, x.h);
     double om_k = om[0];
-        Iface lo{0, 0, 0, 0, 0};
+    Iface lo{0, 0, 0, 0, 0};
     double c_prev = 0.0, d_prev = 0.0;
     double Ek = src[0], Ekp1 = src[plane];
     // row k + 1's inputs are loaded while row k is assembled
@@ -629,9 +629,13 @@ __device__ __forceinline__ void column_newton_step(const EnthArgs& a, const Colu
     }
 }
 
-// One column of the smoother.
-__device__ __forceinline__ void column_s(const EnthArgs& a, int col, double* out, double* rowc, double* dpr,
-                                         double* sm, int mode) {
+template <int MINB>
+__global__ void __launch_bounds__(kColSmemThreads, MINB)
+    k_enth_column_s(EnthArgs a, double* out, double* rowc, double* dpr, int mode) {
+    extern __shared__ double sm[];
+    if (stopped(a.done)) return;
+    const int col = blockIdx.x * blockDim.x + threadIdx.x;
+    if (col >= a.ny * a.nx) return;
     const int nz = a.nz;
     const size_t plane = size_t(a.ny) * a.nx;
     const int i = col / a.nx, j = col % a.nx;
@@ -672,19 +676,14 @@ __device__ __forceinline__ void column_s(const EnthArgs& a, int col, double* out
         column_newton_step<false>(a, x, cl, hc, ct, cs, E, El, C, Dp, cps, blockDim.x, it + 1 == a.n_newton, mode);
 }
 
-template <int MINB>
-__global__ void __launch_bounds__(kColSmemThreads, MINB)
-    k_enth_column_s(EnthArgs a, double* out, double* rowc, double* dpr, int mode) {
-    extern __shared__ double sm[];
-    if (stopped(a.done)) return;
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col < a.ny * a.nx) column_s(a, col, out, rowc, dpr, sm, mode);
-}
-
 // ---------------------------------------------------------- layer smoother
 // enthalpy.cu:1129-1258: pointwise Jacobi, delta = -r / J_kk.  One thread per
 // column walking k.  mode 0 writes delta_E, mode 1 the updated state.
-__device__ __forceinline__ void layer_column(const EnthArgs& a, int col, double* out, int mode) {
+template <int MINB>
+__global__ void __launch_bounds__(kColThreads, MINB) k_enth_layer(EnthArgs a, double* out, int mode) {
+    if (stopped(a.done)) return;
+    const int col = blockIdx.x * blockDim.x + threadIdx.x;
+    if (col >= a.ny * a.nx) return;
     const int nz = a.nz;
     const size_t plane = size_t(a.ny) * a.nx;
     const int i = col / a.nx, j = col % a.nx;
@@ -702,7 +701,7 @@ __device__ __forceinline__ void layer_column(const EnthArgs& a, int col, double*
     double Ek = E[0], Ekp1 = E[plane];
     double Epk = e_pmp(0.0, x.h), Epp = e_pmp(dsig, x.h);
     double om_k = om[0];
-        Iface lo{0, 0, 0, 0, 0};
+    Iface lo{0, 0, 0, 0, 0};
     const bool hadv = (a.flags & kTermHorizAdv) != 0;
     RowIn in = row_inputs(a, x, 0, hadv, true);
     for (int k = 0; k < nz - 1; ++k) {
@@ -733,13 +732,6 @@ __device__ __forceinline__ void layer_column(const EnthArgs& a, int col, double*
     }
     const size_t top = size_t(nz - 1) * plane + x.c;
     out[top] = mode ? E[size_t(nz - 1) * plane] : 0.0;
-}
-
-template <int MINB>
-__global__ void __launch_bounds__(kColThreads, MINB) k_enth_layer(EnthArgs a, double* out, int mode) {
-    if (stopped(a.done)) return;
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col < a.ny * a.nx) layer_column(a, col, out, mode);
 }
 
 // ------------------------------------------------------------ omega
