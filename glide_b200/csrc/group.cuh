@@ -236,13 +236,13 @@ struct GResidual {
         residual_tile<R>(a, item_maps<7>(mp), b);
     }
 };
-template <class R, bool TR, bool SMOOTH>
+template <class R, bool TR, bool SMOOTH, int SLIDE>
 struct GLinear {
     static constexpr int kMinBlocks = StripBlocks<R, SMOOTH>::n;
     using Args = StripArgs<R>;
     static constexpr int kThreads = 32 * kStripWarps;
     static __device__ __forceinline__ void run(const Args& a, const unsigned char*, GroupBlock b) {
-        linear_strip<R, TR, SMOOTH>(a, b);
+        linear_strip<R, TR, SMOOTH, SLIDE>(a, b);
     }
 };
 template <class R, bool TR>

@@ -1141,6 +1141,19 @@ struct Solver : SolverBase {
         return dim3(cols, (q.a.ny + per_block - 1) / per_block);
     }
 
+    // grouped launches merge by this: transposed, linear sliding
+    static int strip_variant(const Lin& L, const StripArgs<R>& q) {
+        return (L.tr ? 1 : 0) | (q.a.p.m == R(1) ? 2 : 0);
+    }
+
+    template <bool SMOOTH>
+    void launch_strip(const Lin& L, const StripArgs<R>& q, dim3 g, cudaStream_t s) {
+        with_slide_code<R>(q.a.p.m == R(1), [&](auto slide) {
+            if (L.tr) k_linear_strip<R, true, SMOOTH, slide()><<<g, 32 * kStripWarps, 0, s>>>(q);
+            else k_linear_strip<R, false, SMOOTH, slide()><<<g, 32 * kStripWarps, 0, s>>>(q);
+        });
+    }
+
     void lin_op(int l, double dt, const Lin& L, const int* out, const int* sub, bool use_forcing, bool norms,
                 bool ref_rows, cudaStream_t s, int jvp_flags = GLIDE_USE_MASK) {
         StripArgs<R> q = strip_args(l, dt, L, out, sub, use_forcing, norms, ref_rows, jvp_flags);
@@ -1168,9 +1181,8 @@ struct Solver : SolverBase {
             return;
         }
         const dim3 g = strip_grid<false>(q);
-        if (!record(G_LINEAR, L.tr ? 1 : 0, g, q, bytes)) {
-            if (L.tr) k_linear_strip<R, true, false><<<g, 32 * kStripWarps, 0, s>>>(q);
-            else k_linear_strip<R, false, false><<<g, 32 * kStripWarps, 0, s>>>(q);
+        if (!record(G_LINEAR, strip_variant(L, q), g, q, bytes)) {
+            launch_strip<false>(L, q, g, s);
             counted(L.tr ? "vjp" : "jvp", bytes);
         }
         if (norms) finish_norms(int(g.x * g.y), s);
@@ -1263,9 +1275,8 @@ struct Solver : SolverBase {
             if (keep_residual && k == n - 1) {
                 q.a.o_u = v.a[L.r[0]]; q.a.o_v = v.a[L.r[1]]; q.a.o_H = v.a[L.r[2]];
             }
-            if (record(G_SMOOTH, L.tr ? 1 : 0, g, q, bytes)) continue;
-            if (L.tr) k_linear_strip<R, true, true><<<g, 32 * kStripWarps, 0, s>>>(q);
-            else k_linear_strip<R, false, true><<<g, 32 * kStripWarps, 0, s>>>(q);
+            if (record(G_SMOOTH, strip_variant(L, q), g, q, bytes)) continue;
+            launch_strip<true>(L, q, g, s);
             counted("linear_sweep", bytes);
         }
         if (fused == n) return;
@@ -1727,9 +1738,19 @@ struct GroupRun : GroupBase {
             case G_NORMS: return issue_op<GNorms>(L, s);
             case G_RESIDUAL: return issue_op<GResidual<R>>(L, s);
             case G_LINEAR:
-                return v ? issue_op<GLinear<R, true, false>>(L, s) : issue_op<GLinear<R, false, false>>(L, s);
-            case G_SMOOTH:
-                return v ? issue_op<GLinear<R, true, true>>(L, s) : issue_op<GLinear<R, false, true>>(L, s);
+            case G_SMOOTH: {
+                long long issued = 0;
+                with_slide_code<R>((v & 2) != 0, [&](auto slide) {
+                    constexpr int S = slide();
+                    if (L.op == G_LINEAR)
+                        issued = (v & 1) ? issue_op<GLinear<R, true, false, S>>(L, s)
+                                         : issue_op<GLinear<R, false, false, S>>(L, s);
+                    else
+                        issued = (v & 1) ? issue_op<GLinear<R, true, true, S>>(L, s)
+                                         : issue_op<GLinear<R, false, true, S>>(L, s);
+                });
+                return issued;
+            }
             case G_SWEEP: {
                 long long issued = 0;
                 with_sweep_form<R>(v >> 1, [&](auto f) {

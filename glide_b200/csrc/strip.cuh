@@ -10,13 +10,14 @@
 //
 // The 16 x 16 tile form this replaces evaluated every face flux and most
 // stresses twice (the transposed product 17 whole rows per cell), read each
-// value from shared memory up to nine times and issued about a thousand
-// instructions per cell for the Jacobian product; the march needs about a
-// third.  What bounds it now is the dependent chain of a row step (loads one
-// row ahead, 16 shuffles, one cube root) at 16 to 20 warps per SM.  Measured at
-// 2048^2: J e in binary32 155 -> 93 us, J^T lambda 264 -> 93 us, in binary64
-// 535 -> 213 us; a smoother sweep (product and block solve) in binary32 225 ->
-// 182 us, of the adjoint 393 -> 168 us, where its bytes alone take 76 and 100.
+// value from shared memory up to nine times and issued about 1050 instructions
+// per owned cell for the Jacobian product; the march issues about 540.  What
+// bounds it now is the dependent chain of a row step (loads one row ahead, 16
+// shuffles, one cube root) at 16 to 20 warps per SM.  Measured at 2048^2: J e in
+// binary32 139 -> 93 us, J^T lambda 264 -> 93 us, in binary64 243 -> 135 and 500 ->
+// 134 us; a smoother sweep (product and block solve) in binary32 225 -> 182 us, of
+// the adjoint 393 -> 168 us, where its bytes alone take 78 and 103 at the measured
+// 6.46 TB/s.
 //
 // Both directions of the coupled operator run here:
 //   TR = false: J e, the exact derivative of the residual rows along e with
@@ -34,6 +35,8 @@
 // Lanes at the strip's edges only feed their neighbours: the stresses reach
 // two columns to the left and right, a face update one cell further to the left.
 #pragma once
+
+#include <type_traits>
 
 #include "adjoint_kernels.cuh"
 
@@ -84,33 +87,20 @@ __device__ __forceinline__ double pow_small(double q, double e) {
     return fma(x, r_low, x) * __hiloint2double((int(n) + 1023) << 20, 0);
 }
 
-// Two powers of one exponent.  Each pow() is a chain of some 150 dependent
-// operations behind a call of its own; these two chains are shorter and overlap.
+// Two powers of one exponent, in line so that their chains overlap: pow() is some
+// 150 dependent operations behind a call of its own.
 struct PowPair { double a, b; };
-__device__ __forceinline__ PowPair pow_two(double x, double y, double e) {
+__device__ __forceinline__ PowPair pow_pair(double x, double y, double e) {
     constexpr double lo = 1e-280, up = 1e280;  // 2^n stays a normal number
     if (fabs(e) <= 1.0 && x > lo && x < up && y > lo && y < up) return {pow_small(x, e), pow_small(y, e)};
-    return {pow(x, e), pow(y, e)};
+    return {pow_general(x, e), pow_general(y, e)};
 }
 
 // d q^e / dq from the power itself.  At q = 0 the quotient says nothing (0 / 0
 // where the derivative is finite).
-template <class P>
-__device__ __forceinline__ double pow_slope(double q, double pw, double e, P&& power) {
-    return q > 0.0 ? e * pw / q : e * power(q, e - 1.0);
+__device__ __forceinline__ double pow_slope(double q, double pw, double e) {
+    return q > 0.0 ? e * pw / q : e * pow_general(q, e - 1.0);
 }
-
-// The powers of a row step's two faces with their derivatives, out of line so that
-// linear sliding keeps its registers: all four for the smoother (the derivatives in
-// line cost it 1 % with m = 1), the powers for the product, where a result that
-// comes back on the stack costs more (J e with m = 1 at 2048^2: 219 us, 273 so).
-struct SlidePair { double a, da, b, db; };
-__device__ __noinline__ inline SlidePair slide_pair(double x, double y, double e) {
-    const PowPair p = pow_two(x, y, e);
-    auto power = [](double q, double k) { return pow(q, k); };
-    return {p.a, pow_slope(x, p.a, e, power), p.b, pow_slope(y, p.b, e, power)};
-}
-__device__ __noinline__ inline PowPair pow_pair(double x, double y, double e) { return pow_two(x, y, e); }
 
 // The neighbouring lanes' values.  All 32 lanes must call: never inside a
 // conditional expression or a branch that is not uniform over the warp.
@@ -137,7 +127,14 @@ struct StripRow {
     R u, v, eu, ev, H, phi, bed, beta, B, eH, mask;
 };
 
-template <class R, bool TR, bool SMOOTH, class BLK>
+// What is compiled for the sliding law.  Binary64 has a kernel for linear sliding
+// and one for the rest: the power's code in one kernel for both cost the product 90
+// bytes of spills at its 168 registers (J e with m = 1: 219 us at 2048^2, 135 on
+// its own; 53 and 35 at 1000 x 760).  In binary32 the power is cheap and one
+// kernel decides as it runs.
+enum SlideCode { kSlideLinear, kSlidePower, kSlideEither };
+
+template <class R, bool TR, bool SMOOTH, int SLIDE, class BLK>
 __device__ __forceinline__ void linear_strip(const StripArgs<R>& q, BLK blk) {
     constexpr int HL = StripShape<SMOOTH>::kLeft, W = StripShape<SMOOTH>::kCols;
     const VjpArgs<R>& a = q.a;
@@ -147,7 +144,8 @@ __device__ __forceinline__ void linear_strip(const StripArgs<R>& q, BLK blk) {
     const int j = int(blk.x()) * W - HL + lane;
     const int ra = (int(blk.y()) * kStripWarps + wp) * q.rows, rb = min(ra + q.rows, ny);
     const bool ref_rows = (q.mode & 1) != 0, use_mask = TR || SMOOTH || (q.mode & 2) == 0;
-    const bool linear = p.m == R(1), calving = p.calving_rate != R(0), f = a.use_forcing != 0;
+    const bool linear = SLIDE == kSlideEither ? p.m == R(1) : SLIDE == kSlideLinear;
+    const bool calving = p.calving_rate != R(0), f = a.use_forcing != 0;
     const R dxi = p.dxi, hdx = R(0.5) * p.dxi;
     const unsigned ju = unsigned(clampi(j, 0, nx)), jc = unsigned(clampi(j, 0, nx - 1));
     const unsigned pu = unsigned(a.u.pitch), pc = unsigned(a.H.pitch);  // v and cell arrays share a pitch
@@ -258,22 +256,17 @@ __device__ __forceinline__ void linear_strip(const StripArgs<R>& q, BLK blk) {
                     // face t row t and, with TR, the v faces t and t + 1.  Four calls
                     // of pow() in every step, two powers and two derivatives, had made
                     // J e with m = 1/3 slower than the 16 x 16 tiles: 51 us at 512^2,
-                    // now 31 (tiles 31); 474, now 332, at 2048^2 (353); 16.4, now 10.3,
-                    // at 64^2 (12.3).  J^T lambda 50 -> 33 at 512^2 (60).
+                    // now 31 (tiles 31); 474, now 322, at 2048^2 (353); 16.4, now 10.6,
+                    // at 64^2 (12.3).  J^T lambda 49 -> 32 at 512^2 (60), 449 -> 298 at
+                    // 2048^2 (825).
                     hu = hv = 0;
                     if (TR || (t >= first && (SMOOTH || t < rb))) {
-                        SlidePair w;
-                        if constexpr (SMOOTH) {
-                            w = slide_pair(qu, qv, e);
-                        } else {
-                            const PowPair pw = pow_pair(qu, qv, e);
-                            w = {pw.a, pow_slope(qu, pw.a, e, pow_general<double>), pw.b,
-                                 pow_slope(qv, pw.b, e, pow_general<double>)};
-                        }
-                        ru -= (beu * (R(2) * w.da * u0 * u0 + w.a) + p.water_drag) * eu0;
-                        rv -= (bev * (R(2) * w.db * v0 * v0 + w.b) + p.water_drag) * ev0;
-                        hu = -beu * (R(0.5) * w.da * u0);
-                        hv = -bev * (R(0.5) * w.db * v0);
+                        const PowPair pw = pow_pair(qu, qv, e);
+                        const R dpu = pow_slope(qu, pw.a, e), dpv = pow_slope(qv, pw.b, e);
+                        ru -= (beu * (R(2) * dpu * u0 * u0 + pw.a) + p.water_drag) * eu0;
+                        rv -= (bev * (R(2) * dpv * v0 * v0 + pw.b) + p.water_drag) * ev0;
+                        hu = -beu * (R(0.5) * dpu * u0);
+                        hv = -bev * (R(0.5) * dpv * v0);
                     }
                 } else {
                     const R dpu = e * pow_general(qu, e - R(1)), dpv = e * pow_general(qv, e - R(1));
@@ -404,15 +397,23 @@ __device__ __forceinline__ void linear_strip(const StripArgs<R>& q, BLK blk) {
     }
 }
 
+// f(the SLIDE to launch, as an integral constant)
+template <class R, class F>
+void with_slide_code(bool linear, F&& f) {
+    if constexpr (sizeof(R) == 4) f(std::integral_constant<int, kSlideEither>{});
+    else if (linear) f(std::integral_constant<int, kSlideLinear>{});
+    else f(std::integral_constant<int, kSlidePower>{});
+}
+
 template <class R, bool SMOOTH>
 struct StripBlocks {
     // resident blocks per SM the registers are fitted to
     static constexpr int n = sizeof(R) == 8 ? (SMOOTH ? 2 : 3) : (SMOOTH ? 4 : 5);
 };
 
-template <class R, bool TR, bool SMOOTH>
+template <class R, bool TR, bool SMOOTH, int SLIDE>
 __global__ void __launch_bounds__(32 * kStripWarps, StripBlocks<R, SMOOTH>::n) k_linear_strip(StripArgs<R> q) {
-    linear_strip<R, TR, SMOOTH>(q, SoloBlock{});
+    linear_strip<R, TR, SMOOTH, SLIDE>(q, SoloBlock{});
 }
 
 }  // namespace glide
