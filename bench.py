@@ -347,22 +347,24 @@ def run_kernels(a):
 # binary32 fine-level kernels on the 2048^2 workload, from one ncu capture of
 # `python bench.py --mode kernels` on a B200 (the command and the figures are
 # in profiles/ssa_kernels_fp32_2048.md, with the commit they were taken at).
-NCU_TRAFFIC_2048_FP32 = {"k_residual": 222.868e6, "k_jvp": 218.683e6, "k_block_factor": 305.240e6,
-                         "k_block_sweep": 356.349e6, "k_vanka_sweep": 245.624e6}
-NCU_TRAFFIC_SOURCE = "profiles/ssa_kernels_fp32_2048.md (ncu, build e3ba9a8)"
+NCU_TRAFFIC_2048_FP32 = {"k_residual": 222.429e6, "k_linear_strip product": 230.156e6, "k_block_factor": 305.354e6,
+                         "k_linear_strip smoother": 524.206e6, "k_vanka_sweep": 244.017e6}
+NCU_TRAFFIC_SOURCE = "profiles/ssa_kernels_fp32_2048.md (ncu, build f98d377)"
 
 
 def kernel_roofline(a, h, stream, fields=None, probe=False):
     """Time the step's hot kernels alone on the step-start state, in the
     precision the step runs them in (binary32 for the mixed form's smoother
-    and tangent operator), with CUDA events: the fused fine-level Vanka
-    sweep, the Jacobian-vector product and the residual.  Algorithmic bytes (N = fine cells, s = bytes per value): residual 15 N s
+    and tangent operator), with CUDA events: the residual, the Jacobian
+    product, the tangent smoother's block factorisation and its fused sweep,
+    and the fused fine-level Vanka sweep.  Algorithmic bytes (N = fine cells,
+    s = bytes per value, F = bytes of a cell's stored factors): residual 15 N s
     (u, v, H, phi, mask, bed, B, beta, gamma, three forcing arrays read, three
-    rows written); the JVP as timed here, without forcing, 14 N s (u, v, H,
+    rows written); the product as timed here, without forcing, 14 N s (u, v, H,
     phi, mask, bed, beta, B and the direction read, three rows written); the
-    fused Vanka sweep 15 N s; the tangent smoother's block factorisation 34 N s
-    (state read, 25 factor planes written) and its block sweep 34 N s (25
-    factors, residual and unknowns read, unknowns written)."""
+    factorisation 9 N s + N F (state read, factors written); the smoother's
+    sweep 17 N s + N F (the product's state, the unknowns, the forcing and the
+    factors read, the unknowns written); the Vanka sweep 15 N s."""
     import torch
     from glide_b200.hierarchy import Hierarchy
     prec = "fp32" if a.precision in ("mixed", "fp32") else "fp64"
@@ -396,22 +398,22 @@ def kernel_roofline(a, h, stream, fields=None, probe=False):
         k.residual(0, a.dt, 8)
         k.jvp(0, a.dt, reference_rows=False)
         k.block_factor(0, a.dt)
-        k.block_sweep(0, a.dt)
+        k.fused_sweeps(0, a.dt)
         k.vanka_sweep(0, a.dt, 1)
         torch.cuda.synchronize()
     # state-preserving kernels first, then the sweep (which moves the state)
-    kernels = [("k_residual", lambda: k.residual(0, a.dt, 8), 15 * n * itemsize),
-               ("k_jvp", lambda: k.jvp(0, a.dt, reference_rows=False), 14 * n * itemsize)]
+    kernels = [("k_residual", lambda: k.residual(0, a.dt, 8), 15 * n * itemsize, 1),
+               ("k_linear_strip product", lambda: k.jvp(0, a.dt, reference_rows=False), 14 * n * itemsize, 1)]
     # the block factors: 25 values per cell, in 13 bfloat16 pairs (52 bytes)
     # under the binary32 tangent smoother
     fbytes = 52 if itemsize == 4 else 25 * itemsize
-    kernels += [("k_block_factor", lambda: k.block_factor(0, a.dt), (9 * itemsize + fbytes) * n),
-                ("k_block_sweep", lambda: k.block_sweep(0, a.dt), (9 * itemsize + fbytes) * n)]
-    kernels += [("k_vanka_sweep", lambda: k.vanka_sweep(0, a.dt, 1), 15 * n * itemsize)]
-    for name, fn, nbytes in kernels:
+    kernels += [("k_block_factor", lambda: k.block_factor(0, a.dt), (9 * itemsize + fbytes) * n, 1),
+                ("k_linear_strip smoother", lambda: k.fused_sweeps(0, a.dt), (17 * itemsize + fbytes) * n, 2)]
+    kernels += [("k_vanka_sweep", lambda: k.vanka_sweep(0, a.dt, 2), 15 * n * itemsize, 2)]
+    for name, fn, nbytes, launches in kernels:
         fn()
         fn()
-        ms = event_time(fn, 10, stream)
+        ms = event_time(fn, 10, stream) / launches
         gbs = nbytes / (ms * 1e-3) / 1e9
         traffic = NCU_TRAFFIC_2048_FP32.get(name) if (a.size == 2048 and prec == "fp32") else None
         out[name] = {"launch_ms": ms, "algorithmic_bytes": nbytes, "achieved_gbs": gbs, "frac": gbs / peak,
@@ -668,7 +670,7 @@ def run_ours(a, rank, world):
             shutil.rmtree(tmp, ignore_errors=True)
 
     # the largest share of the step's device time (launch list of one step)
-    dom = "k_jvp"
+    dom = "k_linear_strip smoother"
     kd = kernels[dom]
     res = {
         "metric": METRIC,

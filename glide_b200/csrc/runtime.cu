@@ -1314,13 +1314,17 @@ struct Solver : SolverBase {
 
     void adj_sweeps(int l, double dt, int n, cudaStream_t s) { lin_sweeps(l, dt, n, adj_sys(), s); }
 
-    // one launch of the linear smoother's block factorisation (part 0) or of
-    // its block sweep on the current residual (part 1), nothing else
+    // the linear smoother's launches alone: block factorisation (part 0), block
+    // sweep on the current residual (part 1), two fused sweeps (part 2)
     void block_part(int l, double dt, bool adjoint, int part, cudaStream_t s) {
         ensure_blocks();
         const Lin L = adjoint ? adj_sys() : tan_sys();
         if (part == 0) {
             block_factor(l, dt, L, s);
+            return;
+        }
+        if (part == 2) {
+            lin_sweeps(l, dt, 2, L, s, false);
             return;
         }
         BlockArgs<R> a = block_args(l, dt, L);
@@ -2427,7 +2431,7 @@ int glide_launch_count(glide_handle h, long long* count) {
 
 int glide_block_smoother_part(glide_handle h, int level, double dt, int adjoint, int part, void* stream) {
     return guarded([&] {
-        if (part < 0 || part > 1) fail(GLIDE_ERR_ARG, "part must be 0 (factorisation) or 1 (sweep)");
+        if (part < 0 || part > 2) fail(GLIDE_ERR_ARG, "part must be 0 (factorisation), 1 (sweep) or 2 (fused sweeps)");
         dispatch(h, [&](auto& s) {
             s.check_level(level);
             s.block_part(level, dt, adjoint != 0, part, S(stream));

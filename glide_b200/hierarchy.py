@@ -281,6 +281,10 @@ class Hierarchy:
         """One launch of the linear smoother's block sweep alone."""
         call("glide_block_smoother_part", self._h, int(level), float(dt), int(bool(adjoint)), 1, _stream_ptr())
 
+    def fused_sweeps(self, level: int, dt: float, adjoint: bool = False):
+        """Two fused sweeps of the linear smoother (product and block solve in one launch each)."""
+        call("glide_block_smoother_part", self._h, int(level), float(dt), int(bool(adjoint)), 2, _stream_ptr())
+
     def adjoint_sweep(self, level: int, dt: float, n: int):
         call("glide_adjoint_sweep", self._h, int(level), float(dt), int(n), _stream_ptr())
 
