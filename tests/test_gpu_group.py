@@ -185,6 +185,9 @@ def test_odd_sweep_counts_in_a_group(precision):
 
     def members():
         out = _members(precision)[:3]
+        h = out[1].mg.hierarchy  # one member slides nonlinearly: kernels of its own in binary64
+        h.set_phys(-1, m=1.0 / 3.0)
+        h.set("beta", 0, 20.0 * h.get("beta", 0), restrict_down=True)
         for m in out:
             apply_schedule(m, CANDIDATES["fast"])
             for which in (False, True, 2):

@@ -78,9 +78,9 @@ def test_compute_jvp_flags_match_reference(tag, kw):
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_jvp_tma_staging_equals_scalar_staging(precision):
-    """The JVP's halo tiles staged by TMA bulk copies (edge tiles fixed up to
-    replicated edge values) give bit-identical results to clamped per-thread
-    loads, on a grid whose tiles are ragged on the right and bottom edges."""
+    """The product is marched from global memory and does not depend on how
+    other kernels stage their tiles (the tiled product of fixed-cycle mixed
+    solves does: tests/test_gpu_fixed_cycles.py)."""
     from cases import random_state
     st = random_state(88, 70, seed=21)
     out = []
@@ -104,9 +104,8 @@ def test_jvp_tma_staging_equals_scalar_staging(precision):
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_vjp_tma_staging_equals_scalar_staging(precision):
-    """The transpose product's two-cell-halo tiles staged by TMA (24-row
-    boxes in binary32, 22-row in binary64, edge tiles fixed up) give
-    bit-identical results to clamped per-thread loads on ragged tiles."""
+    """As above for the transposed product; its 24- and 22-row boxes are staged
+    both ways in the fixed-cycle mixed solves."""
     from cases import random_state
     st = random_state(88, 70, seed=22)
     out = []
