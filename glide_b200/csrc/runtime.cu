@@ -192,35 +192,35 @@ struct RecOp {
 // Blocks of whole groups of four warps fill the four register files evenly
 // (288-thread blocks left a quarter of them idle).  On small grids the sweep is
 // one latency chain, which the smaller blocks shorten; on large ones it is bound
-// by throughput and by how full the last wave is.
+// by throughput, of which 8 x 16 threads with 7 x 15 owned cells waste 18 %, 16 x
+// 16 with 15 x 15 12 %.  In between, how full the last wave is decides, and that
+// moves with the ice: no shape is best there.
 //
-// Binary64 (eight sweeps of a dome; 288-thread blocks / 8 x 16 threads, 7 x 15
-// owned cells, at 3 per SM / at 4 / 16 x 16 at 2), m = 1/3: 64^2 1914 / 1323 /
-// 1414 / 1552 us, 192^2 1903 / 1703 / 1815 / 2160, 250^2 2747 / 3085 / 3145 /
-// 2140, 512^2 8934 / 9335 / 9234 / 8696, 2048^2 144 / 146 / 140 / 129 ms.  With
-// the 168 registers of 3 per SM the compiler contracts the power law's sums
-// otherwise, so that a cell's count of local iterations flips at its threshold now
-// and then (up to 2e-2 in that cell's H on a rough state); the others agree with
-// the 288-thread form bit for bit.  So with m != 1: 8 x 16 at 4 per SM on up to one
-// wave of 3 per SM (444 blocks), then 16 x 16.
+// Binary64 (eight sweeps of a dome; 288-thread blocks / 8 x 16 threads at 3 per SM
+// / at 4 / 16 x 16 at 2).  m = 1/3, ice everywhere: 64^2 1914 / 1323 / 1414 / 1552
+// us, 192^2 1903 / 1703 / 1815 / 2160, 512^2 8934 / 9335 / 9543 / 8696, 1024^2
+// 36.4 / 37.2 / 35.7 / 33.1 ms; margins without ice: 256^2 2740 / 1776 / 2234 /
+// 2157 us, 416^2 5074 / 4546 / 4035 / 4107, 640^2 9702 / 8666 / 8417 / 8009.  m =
+// 1: 64^2 798 / 503 / 583 / 651, 512^2 3792 / 3865 / 3922 / 3893, 1024^2 14.5 /
+// 14.5 / 14.5 / 13.8 ms; with margins 224^2 993 / 686 / - / 912 us, 384^2 2015 /
+// 1464 / - / 1637, 640^2 3915 / 3567 / - / 3519.  So 16 x 16 from 2000 blocks of
+// the small shape on (four and a half waves, about 460^2), where it is at worst 1 %
+// behind and up to 8 % ahead; its 128 registers also leave room beside other
+// streams' kernels, which an ensemble's members run (64 mixed members on 16
+// streams, whose fallback cycles are binary64: 7.05 s a step with 8 x 16 at 3 per
+// SM alone, 6.17 so, 6.80 with 288 threads).
 //
-// With m = 1 all agree, and what counts is how many blocks the fullest SM gets:
-// eight sweeps take about 55 us plus 645 for every three 8 x 16 blocks on it (one
-// left over 350, two 560), or 75 plus 855 for every two 16 x 16 blocks (one left
-// over 520): 240^2 1093 / 930 us, 256^2 1212 / 1445, 400^2 2428 / 2267, 704^2 6931
-// / 6413.  The estimate picks, 16 x 16 within 3 %: its 128 registers leave room
-// beside other streams' kernels, which an ensemble's members run (64 mixed
-// members on 16 streams, whose fallback cycles are binary64: 7.05 s a step with 8
-// x 16 alone, 6.06 so, 6.80 with 288 threads).  A 3-V-cycle step of 512^2 / 64^2
-// takes 51.6 / 27.7 ms (288 threads 56.5 / 31.1, 8 x 16 alone 53.2 / 27.7).
+// Below that, 3 per SM with m = 1 and 4 per SM otherwise: with the 168 registers of
+// 3 per SM the compiler contracts the power law's sums otherwise, so that a cell's
+// count of local iterations flips at its threshold now and then (up to 2e-2 in that
+// cell's H on a rough state).  With m = 1 every form here agrees bit for bit with
+// the 288-thread one, with m != 1 those of at most 128 registers do.
 //
-// Binary32, general, 288-thread / 8 x 16 at 5 per SM / 10 x 32 (9 x 31 cells) at
-// 2: m = 1/3 64^2 469 / 340 / 453 us, 128^2 468 / 387 / 452, 512^2 1949 / 2017 /
-// 2001, 768^2 4382 / 4457 / 4328, 2048^2 30.2 / 30.7 / 29.5 ms; a V-cycle of a
-// mixed handle 64^2 6.09 / 5.14 / 6.38 ms, 512^2 19.9 / 19.3 / 20.2, 1024^2 68.9 /
-// 68.7 / 69.4.  So the wide blocks from four waves of the small ones on (4 x 740).
-// In between, one level's sweeps go either way with how the last wave fills (208^2
-// 630 / 464, 272^2 639 / 771, 368^2 1160 / 1146, 480^2 1915 / 1766 us).
+// Binary32, general, has one shape (288-thread / 8 x 16 at 5 per SM / 16 x 16 at
+// 2): m = 1/3 64^2 469 / 340 / 401 us, 128^2 468 / 387 / 393, 512^2 1949 / 2017 /
+// 2061, 1024^2 7.60 / 7.79 / 7.74 ms; with margins 512^2 1403 / 1331 / 1387 us, 1024^2 4.63 / 4.56 /
+// 4.54 ms; a V-cycle of a mixed handle 64^2 6.09 / 5.14 / 5.56 ms, 512^2 19.9 / 19.3 /
+// 20.4, 1024^2 68.9 / 68.7 / 69.6.
 //
 // Binary32, linear (600 x 424, 2 V-cycles): 8 x 16 at 5 per SM 9.36 ms, at 3 or
 // 4 per SM 9.74.
@@ -231,8 +231,9 @@ static void with_sweep_form(int form, F&& f) {
     switch (form) {
         case S_GENERAL_1: f(SweepForm<false, wide ? 8 : 16, 16, wide ? 2 : 1>{}); break;
         case S_GENERAL_2: f(SweepForm<false, 8, 16, wide ? 3 : 5>{}); break;
+        // binary64 alone has the next two
         case S_GENERAL_POW: f(SweepForm<false, 8, 16, wide ? 4 : 5>{}); break;
-        case S_GENERAL_WIDE: f(SweepForm<false, wide ? 16 : 10, wide ? 16 : 32, 2>{}); break;
+        case S_GENERAL_WIDE: f(SweepForm<false, wide ? 16 : 8, 16, wide ? 2 : 5>{}); break;
         case S_LINEAR: f(SweepForm<!wide, 8, 16, wide ? 3 : 5>{}); break;
         default: fail(GLIDE_ERR_STATE, "unknown sweep form");
     }
@@ -241,16 +242,9 @@ static void with_sweep_form(int form, F&& f) {
 // the shape of the general form at two blocks per SM (figures above)
 template <class R>
 static int general_sweep_form(int ny, int nx, bool linear_sliding) {
-    constexpr int sms = 148;
-    const long long small = (long long)((nx + 14) / 15) * ((ny + 6) / 7);
-    if (sizeof(R) == 4) return small > 4 * sms * 5 ? S_GENERAL_WIDE : S_GENERAL_2;
-    if (!linear_sliding) return small > 3 * sms ? S_GENERAL_WIDE : S_GENERAL_POW;
-    if (small <= 3 * sms) return S_GENERAL_2;
-    const long long wide = (long long)((nx + 14) / 15) * ((ny + 14) / 15);
-    const long long ks = (small + sms - 1) / sms, kw = (wide + sms - 1) / sms;  // blocks of the fullest SM
-    const double t_small = 55 + 645.0 * (ks / 3) + (ks % 3 == 1 ? 350 : ks % 3 == 2 ? 560 : 0);
-    const double t_wide = 75 + 855.0 * (kw / 2) + (kw % 2 ? 520 : 0);
-    return t_wide < 1.03 * t_small ? S_GENERAL_WIDE : S_GENERAL_2;
+    if (sizeof(R) == 4) return S_GENERAL_2;
+    if ((long long)((nx + 14) / 15) * ((ny + 6) / 7) > 2000) return S_GENERAL_WIDE;
+    return linear_sliding ? S_GENERAL_2 : S_GENERAL_POW;
 }
 
 template <class R>
